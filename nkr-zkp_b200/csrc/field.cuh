@@ -7,10 +7,9 @@
 // algebra/fields/fp.hpp:40-42, CUDA mont_t layout operators/cuda/include/fields/
 // mont_t.cuh:45).
 //
-// Multiplication is CIOS Montgomery: per limb of b, one carry chain adds the
-// low halves of a*b_i, one adds the high halves, then the reduction by
-// m = t0 * (-p^-1) repeats the pair of chains with the modulus as immediates.
-// Because p < 2^254, the running value stays below 2p and 9 words suffice.
+// Multiplication is row-wise Montgomery with the running value split into an even
+// and an odd accumulator (mont_mul below).  Because p < 2^254, the running value
+// stays below 2^288 and 9 words suffice.
 #pragma once
 
 #include <cstdint>
@@ -270,53 +269,162 @@ __device__ __forceinline__ uint32_t mod_word(int j)
     }
 }
 
-// The library's Montgomery product: CIOS with 64-bit accumulation of the
-// 32 x 32 -> 64 partial products.  On sm_100a it issues fewer multiply-pipe
-// instructions than explicit 32-bit carry chains (mont_mul_cc below) and
-// measures 14% faster in the throughput microbenchmark (nkr_b200_bench_mul);
-// both forms are bit-identical.
-template <class P, int N>
-__device__ __forceinline__ void mont_mul_body(const Fp<P> *const *a, const Fp<P> *const *b,
-                                              Fp<P> *const *r)
+// ---------------------------------------------------------------------------
+// The Montgomery product.  A 32 x 32 -> 64-bit multiply-add with carry in and out
+// is one instruction (a mad.lo / madc.hi pair on two adjacent words), but only
+// when its 64-bit addend sits in one aligned word pair.  Row i of a x b has eight
+// partial products at word offsets 0..7: those of the even words of a go to the
+// accumulator E (pairs at offsets 0, 2, 4, 6), those of the odd words to O (pairs at
+// 1, 3, 5, 7), so every row is four multiply-adds in one carry chain per
+// accumulator, with no 64-bit addition beside them; m p is added the same way.
+// Shifting the running value down one word turns O into the next row's E and E,
+// less its two lowest words, into its O; the word E[1] left over enters the first
+// multiply-add of the next row as its addend, which cannot overflow.
+//
+// Bound: the multiply pipe, which takes a wide multiply-add every 4 cycles per warp
+// (measured 25-32 lanes per SM and cycle): 128 of them are 512 cycles.  Against the
+// form it replaces (one 64-bit sum per partial product, 219 additions on the ALU
+// pipe and 130 more on the multiply pipe): 43.5 -> 63.7e9 products/s in registers,
+// 579 -> 438 ns for one product after another with one warp per scheduler (B200,
+// 1965 MHz).
+// ---------------------------------------------------------------------------
+
+// (x0..x7) += (a0, a2, a4, a6) b at word offsets 0, 2, 4, 6; c += carry out
+__device__ __forceinline__ void eo_mad(uint32_t *x, uint32_t &c, uint32_t a0, uint32_t a2, uint32_t a4,
+                                       uint32_t a6, uint32_t b)
 {
-    uint32_t t[N][10];
+    asm("mad.lo.cc.u32  %0, %9,  %13, %0;\n\t"
+        "madc.hi.cc.u32 %1, %9,  %13, %1;\n\t"
+        "madc.lo.cc.u32 %2, %10, %13, %2;\n\t"
+        "madc.hi.cc.u32 %3, %10, %13, %3;\n\t"
+        "madc.lo.cc.u32 %4, %11, %13, %4;\n\t"
+        "madc.hi.cc.u32 %5, %11, %13, %5;\n\t"
+        "madc.lo.cc.u32 %6, %12, %13, %6;\n\t"
+        "madc.hi.cc.u32 %7, %12, %13, %7;\n\t"
+        "addc.u32       %8, %8, 0;"
+        : "+r"(x[0]), "+r"(x[1]), "+r"(x[2]), "+r"(x[3]), "+r"(x[4]), "+r"(x[5]), "+r"(x[6]),
+          "+r"(x[7]), "+r"(c)
+        : "r"(a0), "r"(a2), "r"(a4), "r"(a6), "r"(b));
+}
+
+// the same where the sum is known to fit eight words
+__device__ __forceinline__ void eo_mad_fit(uint32_t *x, uint32_t a0, uint32_t a2, uint32_t a4, uint32_t a6,
+                                           uint32_t b)
+{
+    asm("mad.lo.cc.u32  %0, %8,  %12, %0;\n\t"
+        "madc.hi.cc.u32 %1, %8,  %12, %1;\n\t"
+        "madc.lo.cc.u32 %2, %9,  %12, %2;\n\t"
+        "madc.hi.cc.u32 %3, %9,  %12, %3;\n\t"
+        "madc.lo.cc.u32 %4, %10, %12, %4;\n\t"
+        "madc.hi.cc.u32 %5, %10, %12, %5;\n\t"
+        "madc.lo.cc.u32 %6, %11, %12, %6;\n\t"
+        "madc.hi.u32    %7, %11, %12, %7;"
+        : "+r"(x[0]), "+r"(x[1]), "+r"(x[2]), "+r"(x[3]), "+r"(x[4]), "+r"(x[5]), "+r"(x[6]), "+r"(x[7])
+        : "r"(a0), "r"(a2), "r"(a4), "r"(a6), "r"(b));
+}
+
+// (x0..x7) += (a0, a2, a4, a6) b + w with one word w; c = carry out
+__device__ __forceinline__ void eo_mad_word(uint32_t *x, uint32_t &c, uint32_t w, uint32_t a0, uint32_t a2,
+                                            uint32_t a4, uint32_t a6, uint32_t b)
+{
+    asm("{\n\t"
+        ".reg .u32 l, h;\n\t"
+        "mad.lo.cc.u32  l,  %9,  %13, %14;\n\t"
+        "madc.hi.u32    h,  %9,  %13, 0;\n\t"
+        "add.cc.u32     %0, %0,  l;\n\t"
+        "addc.cc.u32    %1, %1,  h;\n\t"
+        "madc.lo.cc.u32 %2, %10, %13, %2;\n\t"
+        "madc.hi.cc.u32 %3, %10, %13, %3;\n\t"
+        "madc.lo.cc.u32 %4, %11, %13, %4;\n\t"
+        "madc.hi.cc.u32 %5, %11, %13, %5;\n\t"
+        "madc.lo.cc.u32 %6, %12, %13, %6;\n\t"
+        "madc.hi.cc.u32 %7, %12, %13, %7;\n\t"
+        "addc.u32       %8, 0, 0;\n\t"
+        "}"
+        : "+r"(x[0]), "+r"(x[1]), "+r"(x[2]), "+r"(x[3]), "+r"(x[4]), "+r"(x[5]), "+r"(x[6]),
+          "+r"(x[7]), "=r"(c)
+        : "r"(a0), "r"(a2), "r"(a4), "r"(a6), "r"(b), "r"(w));
+}
+
+// r = x + y on eight words
+__device__ __forceinline__ void add_words(uint32_t *r, const uint32_t *x, const uint32_t *y)
+{
+    asm("add.cc.u32  %0, %8,  %16;\n\t"
+        "addc.cc.u32 %1, %9,  %17;\n\t"
+        "addc.cc.u32 %2, %10, %18;\n\t"
+        "addc.cc.u32 %3, %11, %19;\n\t"
+        "addc.cc.u32 %4, %12, %20;\n\t"
+        "addc.cc.u32 %5, %13, %21;\n\t"
+        "addc.cc.u32 %6, %14, %22;\n\t"
+        "addc.u32    %7, %15, %23;"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+        : "r"(x[0]), "r"(x[1]), "r"(x[2]), "r"(x[3]), "r"(x[4]), "r"(x[5]), "r"(x[6]), "r"(x[7]),
+          "r"(y[0]), "r"(y[1]), "r"(y[2]), "r"(y[3]), "r"(y[4]), "r"(y[5]), "r"(y[6]), "r"(y[7]));
+}
+
+// r = x + y + c on eight words, c = carry out
+__device__ __forceinline__ void add_words_carry(uint32_t *r, const uint32_t *x, const uint32_t *y, uint32_t &c)
+{
+    asm("add.cc.u32  %8, %8,  0xffffffff;\n\t" // carry in
+        "addc.cc.u32 %0, %9,  %17;\n\t"
+        "addc.cc.u32 %1, %10, %18;\n\t"
+        "addc.cc.u32 %2, %11, %19;\n\t"
+        "addc.cc.u32 %3, %12, %20;\n\t"
+        "addc.cc.u32 %4, %13, %21;\n\t"
+        "addc.cc.u32 %5, %14, %22;\n\t"
+        "addc.cc.u32 %6, %15, %23;\n\t"
+        "addc.cc.u32 %7, %16, %24;\n\t"
+        "addc.u32    %8, 0, 0;"
+        : "=&r"(r[0]), "=&r"(r[1]), "=&r"(r[2]), "=&r"(r[3]), "=&r"(r[4]), "=&r"(r[5]), "=&r"(r[6]),
+          "=&r"(r[7]), "+r"(c)
+        : "r"(x[0]), "r"(x[1]), "r"(x[2]), "r"(x[3]), "r"(x[4]), "r"(x[5]), "r"(x[6]), "r"(x[7]),
+          "r"(y[0]), "r"(y[1]), "r"(y[2]), "r"(y[3]), "r"(y[4]), "r"(y[5]), "r"(y[6]), "r"(y[7]));
+}
+
+// E[0..8], O[0..7] += m p with m = E[0] (-p^-1): word offset 0 becomes zero
+template <class P>
+__device__ __forceinline__ void eo_reduce_row(uint32_t *e, uint32_t *o)
+{
+    const uint32_t m = e[0] * P::INV;
+    eo_mad_fit(o, P::P1, P::P3, P::P5, P::P7, m);
+    eo_mad(e, e[8], P::P0, P::P2, P::P4, P::P6, m);
+}
+
+// a b 2^-256 mod p, below a b / 2^256 + p and not reduced further: for inputs
+// below 2p the result is below 1.76 p.  The running value stays below
+// 2^32 (a + p), within nine words for a < 2p.
+template <class P>
+__device__ __forceinline__ void mont_mul(const uint32_t *a, const uint32_t *b, uint32_t *r)
+{
+    uint32_t e[9], o[8];
 #pragma unroll
-    for (int k = 0; k < N; ++k)
-#pragma unroll
-        for (int j = 0; j < 10; ++j) t[k][j] = 0;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-#pragma unroll
-        for (int k = 0; k < N; ++k) {
-            uint64_t c = 0;
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const uint64_t p = uint64_t(a[k]->v[j]) * b[k]->v[i] + t[k][j] + c;
-                t[k][j] = uint32_t(p);
-                c = p >> 32;
-            }
-            uint64_t s = uint64_t(t[k][8]) + c;
-            t[k][8] = uint32_t(s);
-            t[k][9] = uint32_t(s >> 32);
-            const uint32_t m = t[k][0] * P::INV;
-            c = (uint64_t(m) * P::P0 + t[k][0]) >> 32;
-#pragma unroll
-            for (int j = 1; j < 8; ++j) {
-                const uint64_t p = uint64_t(m) * mod_word<P>(j) + t[k][j] + c;
-                t[k][j - 1] = uint32_t(p);
-                c = p >> 32;
-            }
-            s = uint64_t(t[k][8]) + c;
-            t[k][7] = uint32_t(s);
-            t[k][8] = t[k][9] + uint32_t(s >> 32);
-        }
+    for (int j = 0; j < 4; ++j) {
+        const uint64_t x = uint64_t(a[2 * j]) * b[0], y = uint64_t(a[2 * j + 1]) * b[0];
+        e[2 * j] = uint32_t(x);
+        e[2 * j + 1] = uint32_t(x >> 32);
+        o[2 * j] = uint32_t(y);
+        o[2 * j + 1] = uint32_t(y >> 32);
     }
+    e[8] = 0;
+    eo_reduce_row<P>(e, o);
 #pragma unroll
-    for (int k = 0; k < N; ++k) {
+    for (int i = 1; i < 8; ++i) {
+        uint32_t ne[9], no[8];
+        const uint32_t w = e[1];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) r[k]->v[i] = t[k][i];
-        reduce_once<P>(r[k]->v);
+        for (int j = 0; j < 8; ++j) ne[j] = o[j];
+#pragma unroll
+        for (int j = 0; j < 7; ++j) no[j] = e[j + 2];
+        no[7] = 0;
+        eo_mad_fit(no, a[1], a[3], a[5], a[7], b[i]);
+        eo_mad_word(ne, ne[8], w, a[0], a[2], a[4], a[6], b[i]);
+        eo_reduce_row<P>(ne, no);
+#pragma unroll
+        for (int j = 0; j < 9; ++j) e[j] = ne[j];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) o[j] = no[j];
     }
+    add_words(r, e + 1, o);
 }
 
 // Operands travel by value: an out-of-line call (NKR_FIELD_MUL_OUTLINE) then
@@ -326,14 +434,14 @@ template <class P>
 __device__ NKR_MUL_ATTR Fp<P> operator*(Fp<P> a, Fp<P> b)
 {
     Fp<P> r;
-    const Fp<P> *pa[1] = {&a}, *pb[1] = {&b};
-    Fp<P> *pr[1] = {&r};
-    mont_mul_body<P, 1>(pa, pb, pr);
+    mont_mul<P>(a.v, b.v, r.v);
+    reduce_once<P>(r.v);
     return r;
 }
 
-// The same product with explicit PTX carry chains (two chains per limb of b
-// for the low / high halves, then the reduction pair); kept for comparison.
+// The same product with one accumulator and separate carry chains for the low and
+// the high halves of every row (two half products each, none of which pairs up
+// into a wide multiply-add); kept for comparison.
 template <class P>
 __device__ __forceinline__ Fp<P> mont_mul_cc(const Fp<P> &a, const Fp<P> &b)
 {
@@ -449,48 +557,63 @@ __device__ __forceinline__ Fq2 sqr(const Fq2 &a)
 }
 
 namespace lazy {
-// 256 x 256 -> 512-bit schoolbook product, 64-bit accumulation of the partial
-// products (t[16], little-endian words)
+// 256 x 256 -> 512-bit schoolbook product t[16] (little-endian words): even and odd
+// accumulators as in mont_mul, kept in place.  The chain of row i that starts at
+// offset k ends with its carry at offset k + 8, a word no earlier chain has
+// reached except by its own carry.
 __device__ __forceinline__ void mul_wide(const uint32_t *a, const uint32_t *b, uint32_t *t)
 {
+    uint32_t e[18], o[18]; // o[k] holds word offset k + 1
 #pragma unroll
-    for (int j = 0; j < 16; ++j) t[j] = 0;
+    for (int j = 0; j < 18; ++j) e[j] = o[j] = 0;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        uint64_t c = 0;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const uint64_t p = uint64_t(a[j]) * b[i] + t[i + j] + c;
-            t[i + j] = uint32_t(p);
-            c = p >> 32;
-        }
-        t[i + 8] = uint32_t(c);
+    for (int i = 0; i < 8; i += 2) {
+        eo_mad(e + i, e[i + 8], a[0], a[2], a[4], a[6], b[i]);
+        eo_mad(o + i, o[i + 8], a[1], a[3], a[5], a[7], b[i]);
+        eo_mad(o + i, o[i + 8], a[0], a[2], a[4], a[6], b[i + 1]);
+        eo_mad(e + i + 2, e[i + 10], a[1], a[3], a[5], a[7], b[i + 1]);
     }
+    // t = e + 2^32 o: words 1..8, the carry, words 9..15
+    uint32_t c = 0;
+    t[0] = e[0];
+    uint32_t hi[8]; // words 9..16; the product has none at 16
+    add_words_carry(t + 1, e + 1, o, c);
+    add_words_carry(hi, e + 9, o + 8, c);
+#pragma unroll
+    for (int j = 0; j < 7; ++j) t[9 + j] = hi[j];
 }
 
-// Montgomery reduction T R^-1 mod p of a 512-bit T < p R (R = 2^256): eight
-// word rows clear t[0..7]; the row carry out of t[i + 8] enters row i + 1.  The
-// result is below 2p before the final conditional subtraction.
-__device__ __forceinline__ Fq redc_wide(uint32_t *t)
+// Montgomery reduction T R^-1 mod p of a 512-bit T < p R (R = 2^256): the low half is
+// reduced as in mont_mul (the result is at most p) and added to the high half,
+// below 2p before the final conditional subtraction.
+__device__ __forceinline__ Fq redc_wide(const uint32_t *t)
 {
-    uint32_t hi = 0;
+    uint32_t e[9], o[8];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const uint32_t m = t[i] * FqParams::INV;
-        uint64_t c = (uint64_t(m) * FqParams::P0 + t[i]) >> 32;
+    for (int j = 0; j < 8; ++j) e[j] = t[j], o[j] = 0;
+    e[8] = 0;
+    eo_reduce_row<FqParams>(e, o);
 #pragma unroll
-        for (int j = 1; j < 8; ++j) {
-            const uint64_t p = uint64_t(m) * mod_word<FqParams>(j) + t[i + j] + c;
-            t[i + j] = uint32_t(p);
-            c = p >> 32;
-        }
-        const uint64_t s = uint64_t(t[i + 8]) + c + hi;
-        t[i + 8] = uint32_t(s);
-        hi = uint32_t(s >> 32);
+    for (int i = 1; i < 8; ++i) {
+        uint32_t ne[9], no[8];
+        const uint32_t w = e[1];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) ne[j] = o[j];
+#pragma unroll
+        for (int j = 0; j < 7; ++j) no[j] = e[j + 2];
+        no[7] = 0;
+        const uint32_t m = (ne[0] + w) * FqParams::INV;
+        eo_mad_fit(no, FqParams::P1, FqParams::P3, FqParams::P5, FqParams::P7, m);
+        eo_mad_word(ne, ne[8], w, FqParams::P0, FqParams::P2, FqParams::P4, FqParams::P6, m);
+#pragma unroll
+        for (int j = 0; j < 9; ++j) e[j] = ne[j];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) o[j] = no[j];
     }
     Fq r;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) r.v[i] = t[8 + i];
+    uint32_t lo[8];
+    add_words(lo, e + 1, o);
+    add_words(r.v, lo, t + 8);
     reduce_once<FqParams>(r.v);
     return r;
 }
@@ -533,8 +656,8 @@ __device__ __forceinline__ Fq2L sqr(const Fq2L &a) { return sqr(static_cast<cons
 
 // Fq2 product with lazy reduction: the Karatsuba products are formed as 512-bit
 // integers and combined before reduction, 3 schoolbook products and 2
-// Montgomery reductions instead of 3 Montgomery products (18% fewer
-// multiply-pipe instructions):
+// Montgomery reductions instead of 3 Montgomery products (320 wide multiply-adds
+// instead of 384):
 //   c0 = REDC(a0 b0 + p^2 - a1 b1)                          T in [0, 2 p^2)
 //   c1 = REDC((a0 + a1)(b0 + b1) - a0 b0 - a1 b1)           T = a0 b1 + a1 b0 in [0, 2 p^2)
 // with a0 + a1 and b0 + b1 unreduced (< 2p < 2^255) and 2 p^2 < p R, so each

@@ -40,6 +40,31 @@ def test_field_ops_exact(ctx, rng, field, mod):
     assert np.array_equal(ctx.field_op(field, 6, m), canon)
 
 
+@pytest.mark.parametrize("field,mod", [(0, O.R), (1, O.P), (2, O.P)])
+def test_products_of_extreme_words(ctx, field, mod):
+    """Operands whose 32-bit words are all zeros or all ones (every carry chain of the
+    even and odd accumulators full), the modulus's neighbours and the top word's edge."""
+    top = mod >> 224
+    vals = [sum(((w >> j) & 1) * 0xffffffff << (32 * j) for j in range(7)) | (t << 224)
+            for w in range(128) for t in (0, top - 1)]
+    vals += [mod - 1, mod - 2, 1, 2, (1 << 224) - 1, (top - 1) << 224]
+    limbs = np.stack([O.int_to_limbs(v) for v in vals])
+    a = np.repeat(limbs, len(vals), axis=0)
+    b = np.tile(limbs, (len(vals), 1))
+    rinv = pow(1 << 256, -1, mod)
+    want = np.stack([O.int_to_limbs(x * y * rinv % mod) for x in vals for y in vals])
+    if field != 2:
+        assert np.array_equal(ctx.field_op(field, 0, a, b), want)
+        return
+    # Fq2: (x + y u)(y + x u) = (x^2 + y^2) u and (x + y u)(x - y u) = x^2 + y^2
+    sq = np.stack([O.int_to_limbs((x * x + y * y) * rinv % mod) for x in vals for y in vals])
+    got = ctx.field_op(2, 0, np.concatenate([a, b], axis=1), np.concatenate([b, a], axis=1))
+    assert not got[:, :4].any() and np.array_equal(got[:, 4:], sq)
+    minus = np.stack([O.int_to_limbs(-y % mod) for _ in vals for y in vals])
+    got = ctx.field_op(2, 0, np.concatenate([a, b], axis=1), np.concatenate([a, minus], axis=1))
+    assert np.array_equal(got[:, :4], sq) and not got[:, 4:].any()
+
+
 def test_fp64_limb_arithmetic_matches_integer_arithmetic(ctx, rng):
     """The MSM's FP64-limb Fq (five 52-bit limbs, R = 2^260; fields 3 and 4) gives
     exactly the integer library's results (fields 1 and 2) on edge and random values."""
