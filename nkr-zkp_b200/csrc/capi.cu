@@ -405,7 +405,6 @@ static int msm_plain(nkr_b200_ctx *ctx, int group, const void *bases, const void
     MsmBases b;
     NKR_TRY(msm_bases_build(b, group, bases, false, n, false, 0, false, st));
     MsmScratch s;
-    s.acc.lane_pairs = true; // an MSM alone: latency-bound reduction levels
     NKR_TRY(msm_scratch_alloc(s, group, b.shape));
     DevBuf ds;
     NKR_TRY(ds.alloc(std::max<uint64_t>(n, 1) * 32, "msm scalars"));
@@ -444,7 +443,6 @@ int nkr_b200_msm_bases_create(nkr_b200_ctx *ctx, int group, const void *bases, u
     NKR_TRY(msm_scratch_alloc(h->scratch, group, h->bases.shape));
     for (auto &e : h->scratch.acc.ev_acc) NKR_CUDA(cudaEventCreate(&e));
     h->scratch.acc.timing = true;
-    h->scratch.acc.lane_pairs = true; // MSMs alone: latency-bound reduction levels
     NKR_TRY(h->scalars.alloc(std::max<uint64_t>(n, 1) * 32, "msm scalars"));
     *out = h.release();
     return NKR_B200_OK;
@@ -498,7 +496,8 @@ int nkr_b200_msm_bases_run(nkr_b200_msm_bases *b, const void *scalars, uint64_t 
         uint32_t entries = 0, tasks = 0;
         const uint32_t nb = b->bases.shape.nb;
         NKR_CUDA(cudaMemcpy(&entries, b->scratch.sort.offsets.as<uint32_t>() + nb, 4, cudaMemcpyDeviceToHost));
-        tasks = uint32_t((uint64_t(entries) + b->bases.shape.k1 - 1) / b->bases.shape.k1);
+        const uint32_t k1 = seg_len(entries, uint32_t(b->bases.shape.k1));
+        tasks = uint32_t((uint64_t(entries) + k1 - 1) / k1);
         b->last.entries = entries;
         b->last.tasks = tasks;
         b->last.window_bits = uint32_t(b->bases.shape.c);

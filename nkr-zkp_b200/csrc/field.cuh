@@ -513,6 +513,78 @@ __device__ Fp<P> inverse(const Fp<P> &a)
 }
 
 // ---------------------------------------------------------------------------
+// FqL: Fq values in [0, 2p), the compute type of the G1 MSM.  A product of two such
+// values is below 1.76 p as it stands (mont_mul), so products skip the conditional
+// subtraction; additions and subtractions work modulo 2p.  Zero tests accept 0 and p.
+// Values are made canonical when they leave for memory (canon()).
+// ---------------------------------------------------------------------------
+struct FqL {
+    uint32_t v[8];
+    FqL() = default;
+    __device__ __forceinline__ FqL(const Fq &c)
+    {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[j] = c.v[j];
+    }
+    __device__ __forceinline__ static FqL zero() { return Fq::zero(); }
+    __device__ __forceinline__ static FqL one() { return Fq::one(); }
+    __device__ __forceinline__ bool is_zero() const // 0 or p
+    {
+        uint32_t x = 0, y = 0;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            x |= v[j];
+            y |= v[j] ^ mod_word<FqParams>(j);
+        }
+        return x == 0 || y == 0;
+    }
+    __device__ __forceinline__ Fq canon() const
+    {
+        Fq r;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) r.v[j] = v[j];
+        reduce_once<FqParams>(r.v);
+        return r;
+    }
+    __device__ __forceinline__ bool operator==(const FqL &o) const { return canon() == o.canon(); }
+    __device__ __forceinline__ bool operator!=(const FqL &o) const { return !(*this == o); }
+};
+
+// 2p as a parameter set: reduce_once<TwoP> and the modular additions below
+struct TwoP {
+    static constexpr uint32_t P0 = 0xb0f9fa8eu, P1 = 0x7841182du, P2 = 0xd0e3951au, P3 = 0x2f02d522u,
+                              P4 = 0x0302b0bbu, P5 = 0x70a08b6du, P6 = 0xc2634053u, P7 = 0x60c89ce5u;
+};
+
+__device__ NKR_MUL_ATTR_FN FqL operator*(FqL a, FqL b)
+{
+    FqL r;
+    mont_mul<FqParams>(a.v, b.v, r.v);
+    return r;
+}
+__device__ __forceinline__ FqL sqr(const FqL &a) { return a * a; }
+__device__ __forceinline__ FqL operator+(const FqL &a, const FqL &b)
+{
+    FqL r;
+    add_words(r.v, a.v, b.v);
+    reduce_once<TwoP>(r.v);
+    return r;
+}
+__device__ __forceinline__ FqL operator-(const FqL &a, const FqL &b)
+{
+    Fp<TwoP> x, y;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) x.v[j] = a.v[j], y.v[j] = b.v[j];
+    x = x - y;
+    FqL r;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) r.v[j] = x.v[j];
+    return r;
+}
+__device__ __forceinline__ FqL neg(const FqL &a) { return FqL::zero() - a; }
+__device__ __forceinline__ FqL dbl(const FqL &a) { return a + a; }
+
+// ---------------------------------------------------------------------------
 // Fq2 = Fq[u] / (u^2 + 1)  (libff alt_bn128_Fq2, non_residue = -1)
 // ---------------------------------------------------------------------------
 struct alignas(32) Fq2 {

@@ -9,91 +9,12 @@
 #include <cstring>
 #include <type_traits>
 
-#include "field52.cuh"
 #include "msm.cuh"
 #include "pairing.cuh" // twist_frobenius: the endomorphism psi of G2
+#include "quad.cuh"
 #include "scan.cuh"
 
 namespace nkr {
-
-// --------------------------------------------------------------------------
-// lane pairs.  The bucket reduction levels are chains of dependent additions
-// run by few threads, so there each addition is computed by two lanes: the
-// curve formulas issue their products in independent pairs (mul2), and a lane
-// pair computes one product of each pair and exchanges the results.  Everything
-// else is computed by both lanes alike, so a pair stays converged.
-// --------------------------------------------------------------------------
-template <class B>
-struct Pair2 : B {
-    using base = B;
-    Pair2() = default;
-    __device__ __forceinline__ Pair2(const B &b) : B(b) {}
-    __device__ __forceinline__ static Pair2 zero() { return B::zero(); }
-    __device__ __forceinline__ static Pair2 one() { return B::one(); }
-};
-template <class B>
-__device__ __forceinline__ Pair2<B> operator+(const Pair2<B> &a, const Pair2<B> &b)
-{
-    return static_cast<const B &>(a) + static_cast<const B &>(b);
-}
-template <class B>
-__device__ __forceinline__ Pair2<B> operator-(const Pair2<B> &a, const Pair2<B> &b)
-{
-    return static_cast<const B &>(a) - static_cast<const B &>(b);
-}
-template <class B>
-__device__ __forceinline__ Pair2<B> operator*(const Pair2<B> &a, const Pair2<B> &b)
-{
-    return static_cast<const B &>(a) * static_cast<const B &>(b);
-}
-template <class B>
-__device__ __forceinline__ Pair2<B> dbl(const Pair2<B> &a) { return dbl(static_cast<const B &>(a)); }
-template <class B>
-__device__ __forceinline__ Pair2<B> sqr(const Pair2<B> &a) { return sqr(static_cast<const B &>(a)); }
-
-__device__ __forceinline__ Fq52 shfl_xor1(unsigned mask, const Fq52 &a)
-{
-    Fq52 r;
-#pragma unroll
-    for (int j = 0; j < 5; ++j) r.l[j] = __shfl_xor_sync(mask, a.l[j], 1);
-    return r;
-}
-__device__ __forceinline__ Fq52L shfl_xor1(unsigned mask, const Fq52L &a)
-{
-    Fq52L r;
-#pragma unroll
-    for (int j = 0; j < 5; ++j) r.l[j] = __shfl_xor_sync(mask, a.l[j], 1);
-    return r;
-}
-__device__ __forceinline__ Fq2 shfl_xor1(unsigned mask, const Fq2 &a)
-{
-    Fq2 r;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        r.c0.v[j] = __shfl_xor_sync(mask, a.c0.v[j], 1);
-        r.c1.v[j] = __shfl_xor_sync(mask, a.c1.v[j], 1);
-    }
-    return r;
-}
-
-// the pair of lanes (2j, 2j + 1) of the calling lane
-__device__ __forceinline__ unsigned pair_mask() { return 3u << ((threadIdx.x & 31u) & 30u); }
-
-// x = a b, y = c d: the even lane computes a b, the odd lane c d
-template <class B>
-__device__ __forceinline__ void mul2(const Pair2<B> &a, const Pair2<B> &b, const Pair2<B> &c,
-                                     const Pair2<B> &d, Pair2<B> &x, Pair2<B> &y)
-{
-    const bool odd = threadIdx.x & 1u;
-    const B m = static_cast<const B &>(odd ? c : a) * static_cast<const B &>(odd ? d : b);
-    const B o = shfl_xor1(pair_mask(), m);
-    x = odd ? o : m;
-    y = odd ? m : o;
-}
-template <class B>
-struct HasPairedMul<Pair2<B>> {
-    static constexpr bool value = true;
-};
 
 namespace {
 
@@ -202,97 +123,31 @@ __global__ void k_scatter(const Fr *__restrict__ canon, uint64_t n, int c, int W
 }
 
 // --------------------------------------------------------------------------
-// storage vs compute.  G1 arithmetic runs on the FP64 pipe (Fq52, R' = 2^260):
-// every G1 MSM buffer (bases, partials, buckets, reduction items) holds R'-domain
-// values in the 8 x 32-bit layout of Fq, converted at entry (bases) and exit
-// (result).  G2 arithmetic stays on the integer pipe (Fq2, R = 2^256): measured,
-// its FP64 form (Fq2 products as three interleaved 52-bit products) needs all 255
-// registers and ran 34% slower at 2^18 points; with the accumulator in shared
-// memory as for G1 (254 registers, bases in R' from prepare, flushes leaving R')
-// the level-1 kernel took 7.96 instead of 3.48 ms.  The same holds for the G2
-// reduction levels alone, although they are latency bound (a 32-bit product is
-// one long carry chain): in the FP64 form they spill 600 B per thread and took
-// 1.81 instead of 1.53 ms at 2^18; with the three Karatsuba products of an Fq2
-// product interleaved in one 32-bit call they took 1.66 ms, no faster.  Moving one
-// Karatsuba product of every Fq2 product to the FP64 pipe ((16 x) y 2^-260 =
-// x y 2^-256) relieves the integer multiply pipe but costs four doublings, limb
-// conversions and spills at 255 registers: the G2 accumulation took 4.01 instead
-// of 3.48 ms at 2^18.
+// storage vs compute.  Every MSM buffer (bases, partials, buckets, reduction items)
+// holds canonical values of Fq or Fq2.  Level 1 computes in FqL (G1, values below 2p)
+// and Fq2 (G2), the levels after it on quads of lanes (quad.cuh) in FqL and Fq2L, the
+// Fq2 product with two reductions instead of three.
 // --------------------------------------------------------------------------
 
 template <class F>
 struct MsmArith;
 template <>
 struct MsmArith<Fq> {
-    using type = Fq52L;
+    using type = FqL;
+    using quad = FqL;
 };
 template <>
 struct MsmArith<Fq2> {
     using type = Fq2;
+    using quad = Fq2L;
 };
 template <class F>
 using CF = typename MsmArith<F>::type;
-
-// Compute type and shape of the bucket reduction levels (first level, block
-// levels, final combination): latency-bound chains of dependent additions, with
-// LANES lanes per item.  G2 computes in the lazily reduced Fq2 product (Fq2L,
-// field.cuh), 128 items per block; an MSM alone (MsmAcc::lane_pairs) runs it on
-// lane pairs (Pair2): at 2^18 points the block levels 1.21 -> 0.85 ms and the
-// first level 0.36 -> 0.28 ms.  Inside a prove the G2 levels overlap the other
-// MSMs' level-1 kernels, and there the pairs' 256-thread blocks, which take a
-// whole SM's registers, cost more than they save (2^20 prove 19.09 vs 18.97 ms),
-// so a prove keeps one lane per item.  G1 keeps one lane per item and 256 items
-// per block: on lane pairs (128 items per block, the register budget of a
-// 256-thread block) its block levels are shorter but its first level takes
-// twice the buckets per pair (2^20 MSM 4.31 vs 4.25 ms; a 2^20 prove 19.16 ms).
 template <class F>
-struct ReduceBase {
-    using type = CF<F>;
-};
-template <>
-struct ReduceBase<Fq2> {
-    using type = Fq2L;
-};
-template <class F, int LANES>
-struct MsmReduceArith {
-    using type = typename std::conditional<LANES == 2, Pair2<typename ReduceBase<F>::type>,
-                                           typename ReduceBase<F>::type>::type;
-    static constexpr int lanes = LANES;
-    static constexpr int items = (LANES == 1 && sizeof(F) == sizeof(Fq)) ? 256 : 128;
-    static constexpr int log2_items = items == 256 ? 8 : 7;
-};
-template <class C>
-struct BaseOf {
-    using type = C;
-};
-template <class B>
-struct BaseOf<Pair2<B>> {
-    using type = B;
-};
+using QF = typename MsmArith<F>::quad;
 
-// G1 buffers hold canonical values; the lazily reduced compute values are
-// canonicalised on the way out
-__device__ __forceinline__ Fq52L msm_in(const Fq &x) { return to52(x); }
-__device__ __forceinline__ Fq msm_out(const Fq52L &x) { return from52(x.canon()); }
-__device__ __forceinline__ Fq52L msm_enter(const Fq52L &x) { return r256_to_r260(x.canon()); }
-__device__ __forceinline__ Fq52L msm_leave(const Fq52L &x) { return r260_to_r256(x.canon()); }
-__device__ __forceinline__ Fq2 msm_in(const Fq2 &x) { return x; }
+__device__ __forceinline__ Fq msm_out(const FqL &x) { return x.canon(); }
 __device__ __forceinline__ Fq2 msm_out(const Fq2 &x) { return x; }
-__device__ __forceinline__ Fq2 msm_enter(const Fq2 &x) { return x; }
-__device__ __forceinline__ Fq2 msm_leave(const Fq2 &x) { return x; }
-
-template <class F>
-__device__ __forceinline__ Xyzz<CF<F>> ldx(const Xyzz<F> &s)
-{
-    return {msm_in(s.x), msm_in(s.y), msm_in(s.zz), msm_in(s.zzz)};
-}
-
-template <class C, class F>
-__device__ __forceinline__ Xyzz<C> ldr(const Xyzz<F> &s)
-{
-    using B = typename BaseOf<C>::type;
-    return {B(msm_in(s.x)), B(msm_in(s.y)), B(msm_in(s.zz)), B(msm_in(s.zzz))};
-}
 
 template <class C>
 __device__ __forceinline__ auto stx(const Xyzz<C> &c) -> Xyzz<decltype(msm_out(c.x))>
@@ -303,7 +158,27 @@ __device__ __forceinline__ auto stx(const Xyzz<C> &c) -> Xyzz<decltype(msm_out(c
 template <class F>
 __device__ __forceinline__ Affine<CF<F>> lda(const Affine<F> &s)
 {
-    return {msm_in(s.x), msm_in(s.y)};
+    return {CF<F>(s.x), CF<F>(s.y)};
+}
+
+// this lane's coordinate of a point in memory, read from L2 (the fix-up levels read
+// what other blocks of their own launch wrote)
+template <class F>
+__device__ __forceinline__ QF<F> quad_ld(const Xyzz<F> *p)
+{
+    union {
+        uint4 w[sizeof(F) / 16];
+        F f;
+    } u;
+    const uint4 *q = reinterpret_cast<const uint4 *>(reinterpret_cast<const F *>(p) + quad_role());
+#pragma unroll
+    for (unsigned j = 0; j < sizeof(F) / 16; ++j) u.w[j] = __ldcg(q + j);
+    return QF<F>(u.f);
+}
+template <class F>
+__device__ __forceinline__ void quad_st(Xyzz<F> *p, const QF<F> &v)
+{
+    reinterpret_cast<F *>(p)[quad_role()] = msm_out(v);
 }
 
 // first index in a[0, n) with a[idx] > x (a nondecreasing)
@@ -345,60 +220,62 @@ __device__ __forceinline__ Pieces bucket_pieces(const uint32_t *offsets, uint32_
     return {t0, t1 - t0 + 1};
 }
 
-// Groups of k2 pieces a bucket still has at a fix-up level whose inputs are
-// spaced `stride` pieces apart (zero once the bucket is complete).
-constexpr unsigned kFixupBlocks = 148 * 8; // grid cap of a fix-up level
-
 // Buckets of at most kSmallPieces pieces are summed where they are consumed
-// (k_reduce_first); only larger ones go through the fix-up levels.
-constexpr uint32_t kSmallPieces = 16;
+// (k_reduce_first); larger ones first go through the fix-up levels (k_fix_up), in
+// groups of kFixGroup pieces.
+constexpr uint32_t kSmallPieces = 4;
+constexpr uint32_t kFixGroup = 4;
+constexpr unsigned kFixupBlocks = 148 * 8; // grid cap of the fix-up kernel
 
-struct LoadLeaders {
-    const uint32_t *offsets;
-    uint32_t k1, stride, k2;
-    __device__ __forceinline__ uint32_t operator()(uint64_t i) const
+// The first-level groups of the large buckets, pushed by level 1, and the arrival
+// counters of the levels above: base[0] counts the items {bucket, group}, base + 4
+// holds them, and base + 4 + 2 cap has one counter per partial slot (zeroed by level 1).
+struct FixList {
+    uint32_t *base;
+    uint32_t cap;
+    __device__ __forceinline__ uint2 *items() const { return reinterpret_cast<uint2 *>(base + 4); }
+    __device__ __forceinline__ uint32_t *counters() const { return base + 4 + 2ull * cap; }
+    __device__ __forceinline__ void push(uint32_t bucket, uint32_t group) const
     {
-        const Pieces pc = bucket_pieces(offsets, uint32_t(i), k1);
-        if (pc.count <= kSmallPieces) return 0u;
-        const uint32_t live = (pc.count + stride - 1) / stride;
-        return live > 1 ? (live + k2 - 1) / k2 : 0u;
+        const uint32_t i = atomicAdd(base, 1u);
+        if (i < cap) items()[i] = {bucket, group};
     }
 };
+// a bucket of more than kSmallPieces pieces has at most pieces / kFixGroup + 1 groups and all
+// buckets together at most 2 segs pieces
+uint32_t fix_cap(uint64_t segs) { return uint32_t(segs + 2); }
+size_t fix_bytes(uint64_t segs) { return 16 + 8ull * fix_cap(segs) + 8 * segs; }
 
-// Level-1 accumulators live in shared memory.  Across the out-of-line product
-// calls of a mixed addition the four accumulator coordinates were live in
-// registers (G1: 40 of the 168 the 3-blocks-per-SM budget allows, with 100 B of
-// spills per thread; G2: 64 of 232, 2 blocks per SM); kept in shared memory and
-// loaded where a product needs them, G1 runs its 3-block budget without spills
-// (1.4% faster at 2^20) and G2 fits 3 blocks per SM in 167 registers without
-// spills (6% faster at 2^18).  Layout: structure of arrays, word w of thread i
-// at w * BS + i, so a warp's accesses are conflict-free.
+// Level-1 accumulators live in shared memory: across the out-of-line product calls of a
+// mixed addition their four coordinates would otherwise stay in registers.  Layout:
+// structure of arrays, word w of thread i at w * BS + i, so a warp's accesses are
+// conflict-free.
 //
-// G1: Fq52L coordinates (5 x 64-bit words, lazily reduced), R' domain throughout.
+// G1: FqL coordinates (8 words, below 2p).
 template <int BS>
-struct SmXyzz52 {
-    using point = Affine<Fq52L>;
-    uint64_t *s; // the block's area + threadIdx.x; 20 words per thread
-    __device__ __forceinline__ Fq52L ld(int f) const
+struct SmXyzzFq {
+    using point = Affine<FqL>;
+    uint32_t *s; // the block's area + threadIdx.x; 32 words per thread
+    __device__ __forceinline__ FqL ld(int f) const
     {
-        Fq52L v;
+        FqL v;
 #pragma unroll
-        for (int j = 0; j < 5; ++j) v.l[j] = s[(f * 5 + j) * BS];
+        for (int j = 0; j < 8; ++j) v.v[j] = s[(f * 8 + j) * BS];
         return v;
     }
-    __device__ __forceinline__ void st(int f, const Fq52L &v) const
+    __device__ __forceinline__ void st(int f, const FqL &v) const
     {
 #pragma unroll
-        for (int j = 0; j < 5; ++j) s[(f * 5 + j) * BS] = v.l[j];
+        for (int j = 0; j < 8; ++j) s[(f * 8 + j) * BS] = v.v[j];
     }
-    __device__ __forceinline__ void set(const Xyzz<Fq52L> &a) const
+    __device__ __forceinline__ void set(const Xyzz<FqL> &a) const
     {
         st(0, a.x);
         st(1, a.y);
         st(2, a.zz);
         st(3, a.zzz);
     }
-    __device__ __forceinline__ Xyzz<Fq> out() const { return stx(Xyzz<Fq52L>{ld(0), ld(1), ld(2), ld(3)}); }
+    __device__ __forceinline__ Xyzz<Fq> out() const { return stx(Xyzz<FqL>{ld(0), ld(1), ld(2), ld(3)}); }
     __device__ __forceinline__ static point load(const Affine<Fq> &p) { return lda(p); }
 };
 
@@ -436,9 +313,8 @@ struct SmXyzzFq2 {
     __device__ __forceinline__ static point load(const Affine<Fq2> &p) { return p; }
 };
 
-// acc + q (madd-2008-s: 8M + 2S) on a shared-memory accumulator, q may be
-// infinity; the products go in the pairs of xyzz_add_affine (G1's paired
-// product)
+// acc + q (madd-2008-s: 8M + 2S) on a shared-memory accumulator, q may be infinity;
+// each product comes right before its first use, which keeps few values live
 template <class Acc, class C>
 __device__ __forceinline__ void sm_add_affine(const Acc &a, const Affine<C> &q)
 {
@@ -448,51 +324,19 @@ __device__ __forceinline__ void sm_add_affine(const Acc &a, const Affine<C> &q)
         a.set({q.x, q.y, C::one(), C::one()});
         return;
     }
-    C u2, s2;
-    mul2(q.x, zz, q.y, a.ld(3), u2, s2);
-    const C p = u2 - a.ld(0);
-    const C r = s2 - a.ld(1);
+    const C p = q.x * zz - a.ld(0);
+    const C r = q.y * a.ld(3) - a.ld(1);
     if (p.is_zero()) {
         a.set(r.is_zero() ? xyzz_from_affine_dbl(q) : Xyzz<C>::inf());
         return;
     }
-    C pp, rr, ppp, qq, y1ppp, ry, t;
-    mul2(p, p, r, r, pp, rr);
-    mul2(p, pp, a.ld(0), pp, ppp, qq);
-    mul2(a.ld(3), ppp, a.ld(1), ppp, t, y1ppp);
-    a.st(3, t);
-    const C ox = rr - ppp - dbl(qq);
-    a.st(0, ox);
-    mul2(r, qq - ox, a.ld(2), pp, ry, t);
-    a.st(2, t);
-    a.st(1, ry - y1ppp);
-}
-
-// The same for G2, whose products are single calls: each product right before
-// its first use keeps fewer values live (167 registers and no spills at the
-// 3-block budget, against 104 B of spills in the paired order)
-template <int BS>
-__device__ __forceinline__ void sm_add_affine(const SmXyzzFq2<BS> &a, const Affine<Fq2> &q)
-{
-    if (q.is_inf()) return;
-    const Fq2 zz = a.ld(2);
-    if (zz.is_zero()) {
-        a.set({q.x, q.y, Fq2::one(), Fq2::one()});
-        return;
-    }
-    const Fq2 p = q.x * zz - a.ld(0);
-    const Fq2 r = q.y * a.ld(3) - a.ld(1);
-    if (p.is_zero()) {
-        a.set(r.is_zero() ? xyzz_from_affine_dbl(q) : Xyzz<Fq2>::inf());
-        return;
-    }
-    const Fq2 pp = sqr(p);
-    const Fq2 ppp = p * pp;
+    const C pp = sqr(p);
+    const C ppp = p * pp;
     a.st(3, a.ld(3) * ppp);
-    const Fq2 qq = a.ld(0) * pp;
-    const Fq2 ox = sqr(r) - ppp - dbl(qq);
+    const C qq = a.ld(0) * pp;
+    const C ox = sqr(r) - ppp - dbl(qq);
     a.st(0, ox);
-    const Fq2 y1ppp = a.ld(1) * ppp;
+    const C y1ppp = a.ld(1) * ppp;
     a.st(1, r * (qq - ox) - y1ppp);
     a.st(2, a.ld(2) * pp);
 }
@@ -501,23 +345,34 @@ __device__ __forceinline__ void sm_add_affine(const SmXyzzFq2<BS> &a, const Affi
 // entries, split into runs at bucket boundaries, so every lane of a warp does
 // the same number of mixed additions whatever the bucket sizes.  A run that is
 // a whole bucket is written to the bucket; the segment's first / last run, when
-// its bucket continues outside the segment, goes to partial slot 2t / 2t + 1.
+// its bucket continues outside the segment, goes to partial slot 2t / 2t + 1.  The
+// segment of every kFixGroup-th piece of a large bucket puts that group on the fix-up
+// list.
 template <class Acc, class F>
 __device__ __forceinline__ void acc_l1_body(const uint32_t *__restrict__ offsets,
                                             const uint32_t *__restrict__ entries,
                                             const Affine<F> *__restrict__ pts, uint32_t nb,
-                                            uint32_t k1, Xyzz<F> *__restrict__ partials,
-                                            Xyzz<F> *__restrict__ buckets, uint32_t t, const Acc &acc)
+                                            uint32_t kmax, Xyzz<F> *__restrict__ partials,
+                                            Xyzz<F> *__restrict__ buckets, const FixList &fix, uint32_t t,
+                                            const Acc &acc)
 {
     using C = decltype(acc.ld(0));
     const uint32_t total = offsets[nb];
+    const uint32_t k1 = seg_len(total, kmax);
     const uint64_t beg64 = uint64_t(t) * k1;
     if (beg64 >= total) return;
+    fix.counters()[2ull * t] = 0;
+    fix.counters()[2ull * t + 1] = 0;
     const uint32_t beg = uint32_t(beg64);
     const uint32_t end = min(beg + k1, total);
     uint32_t b = upper_bound_u32(offsets, nb + 1, beg) - 1; // offsets[b] <= beg < offsets[b + 1]
     uint32_t bstart = offsets[b], bend = offsets[b + 1];
     bool first = true;
+    auto to_partial = [&] {
+        partials[2ull * t + (first ? 0 : 1)] = acc.out();
+        const uint32_t t0 = bstart / k1, pieces = (bend - 1) / k1 - t0 + 1;
+        if (pieces > kSmallPieces && (t - t0) % kFixGroup == 0) fix.push(b, (t - t0) / kFixGroup);
+    };
     acc.set(Xyzz<C>::inf());
     // one flat loop with the same trip count in every lane keeps the additions
     // converged; the flush at a bucket boundary is a short divergent branch
@@ -526,7 +381,7 @@ __device__ __forceinline__ void acc_l1_body(const uint32_t *__restrict__ offsets
             if (bstart >= beg)
                 buckets[b] = acc.out(); // the bucket started and ended inside the segment
             else
-                partials[2ull * t] = acc.out(); // first run, bucket began in an earlier segment
+                to_partial(); // first run, bucket began in an earlier segment
             first = false;
             acc.set(Xyzz<C>::inf());
             // next nonempty bucket: usually adjacent, else search
@@ -548,38 +403,31 @@ __device__ __forceinline__ void acc_l1_body(const uint32_t *__restrict__ offsets
     if (bstart >= beg && bend <= end)
         buckets[b] = acc.out();
     else
-        partials[2ull * t + (first ? 0 : 1)] = acc.out();
+        to_partial();
 }
 
-// Level 1 kernels, 3 blocks of 128 threads per SM.  G1 (FP64 field, paired
-// products passed by value): measured against the compiler's own register
-// choice (184 registers, 2 blocks) and a 4-block budget (128 registers, 124 B of
-// spills), the fastest from 2^16 to 2^20 points, uniform and sparse.  G2 (integer
-// pipe): 167 registers without spills, against 232 at 2 blocks per SM before the
-// accumulator moved to shared memory (a 4-block budget spills 232 B and is no
-// faster).
-__global__ void __launch_bounds__(128, 3) k_acc_l1_g1(const uint32_t *__restrict__ offsets,
+__global__ void __launch_bounds__(128, 4) k_acc_l1_g1(const uint32_t *__restrict__ offsets,
                                                        const uint32_t *__restrict__ entries,
                                                        const Affine<Fq> *__restrict__ pts,
-                                                       uint32_t nb, uint32_t k1,
+                                                       uint32_t nb, uint32_t kmax,
                                                        Xyzz<Fq> *__restrict__ partials,
-                                                       Xyzz<Fq> *__restrict__ buckets)
+                                                       Xyzz<Fq> *__restrict__ buckets, FixList fix)
 {
-    __shared__ uint64_t sm[20 * 128];
-    acc_l1_body(offsets, entries, pts, nb, k1, partials, buckets, blockIdx.x * blockDim.x + threadIdx.x,
-                SmXyzz52<128>{sm + threadIdx.x});
+    __shared__ uint32_t sm[32 * 128];
+    acc_l1_body(offsets, entries, pts, nb, kmax, partials, buckets, fix,
+                blockIdx.x * blockDim.x + threadIdx.x, SmXyzzFq<128>{sm + threadIdx.x});
 }
 
 __global__ void __launch_bounds__(128, 3) k_acc_l1_g2(const uint32_t *__restrict__ offsets,
                                                        const uint32_t *__restrict__ entries,
                                                        const Affine<Fq2> *__restrict__ pts,
-                                                       uint32_t nb, uint32_t k1,
+                                                       uint32_t nb, uint32_t kmax,
                                                        Xyzz<Fq2> *__restrict__ partials,
-                                                       Xyzz<Fq2> *__restrict__ buckets)
+                                                       Xyzz<Fq2> *__restrict__ buckets, FixList fix)
 {
     __shared__ uint32_t sm[64 * 128];
-    acc_l1_body(offsets, entries, pts, nb, k1, partials, buckets, blockIdx.x * blockDim.x + threadIdx.x,
-                SmXyzzFq2<128>{sm + threadIdx.x});
+    acc_l1_body(offsets, entries, pts, nb, kmax, partials, buckets, fix,
+                blockIdx.x * blockDim.x + threadIdx.x, SmXyzzFq2<128>{sm + threadIdx.x});
 }
 
 // Level 1 of several MSMs of one group in one launch (a batch's MSMs, any sizes):
@@ -589,7 +437,8 @@ struct AccItem {
     const uint32_t *offsets, *entries;
     const Affine<F> *pts;
     Xyzz<F> *partials, *buckets;
-    uint32_t nb, k1, first_block;
+    uint32_t *fix_base;
+    uint32_t fix_capacity, nb, kmax, first_block;
 };
 static_assert(sizeof(AccItem<Fq>) <= kMsmAccItemBytes, "work-list item size");
 
@@ -608,75 +457,92 @@ __device__ __forceinline__ AccItem<F> acc_list_item(const AccItem<F> *items, int
     return items[lo];
 }
 
-__global__ void __launch_bounds__(128, 3) k_acc_l1_g1_list(const AccItem<Fq> *items, int n_items)
+__global__ void __launch_bounds__(128, 4) k_acc_l1_g1_list(const AccItem<Fq> *items, int n_items)
 {
-    __shared__ uint64_t sm[20 * 128];
+    __shared__ uint32_t sm[32 * 128];
     const AccItem<Fq> it = acc_list_item(items, n_items);
-    acc_l1_body(it.offsets, it.entries, it.pts, it.nb, it.k1, it.partials, it.buckets,
-                (blockIdx.x - it.first_block) * blockDim.x + threadIdx.x, SmXyzz52<128>{sm + threadIdx.x});
+    acc_l1_body(it.offsets, it.entries, it.pts, it.nb, it.kmax, it.partials, it.buckets,
+                FixList{it.fix_base, it.fix_capacity},
+                (blockIdx.x - it.first_block) * blockDim.x + threadIdx.x, SmXyzzFq<128>{sm + threadIdx.x});
 }
 
 __global__ void __launch_bounds__(128, 3) k_acc_l1_g2_list(const AccItem<Fq2> *items, int n_items)
 {
     __shared__ uint32_t sm[64 * 128];
     const AccItem<Fq2> it = acc_list_item(items, n_items);
-    acc_l1_body(it.offsets, it.entries, it.pts, it.nb, it.k1, it.partials, it.buckets,
+    acc_l1_body(it.offsets, it.entries, it.pts, it.nb, it.kmax, it.partials, it.buckets,
+                FixList{it.fix_base, it.fix_capacity},
                 (blockIdx.x - it.first_block) * blockDim.x + threadIdx.x, SmXyzzFq2<128>{sm + threadIdx.x});
 }
 
-// One group of k2 pieces (spaced `stride` pieces apart) of one bucket; the
-// group's sum goes back into the group's first piece slot, or into the bucket
-// when it was the bucket's last group.
+// The pieces of the large buckets, one launch for all levels: a quad sums a group of
+// kFixGroup pieces into the group's first slot and counts itself in at the parent
+// group; the quad that arrives last (nobody waits) sums the parent's up to kFixGroup
+// children, and so on until the bucket is one piece, which goes to the bucket.  The
+// counter of a parent at level l is that of its (l + 1)-th piece: a parent of at least
+// two children has more than kFixGroup^l pieces, so these exist and differ per level.
+// Every level cost a scan and a launch before (four levels at 2^20 segments), and a
+// group took 16 additions by one thread (130 us); a sparse MSM of 200,003 points
+// spends 364 us less here.
 template <class F>
-__device__ __forceinline__ void acc_up_group(const uint32_t *__restrict__ offsets,
-                                             const uint32_t *__restrict__ lead_off, uint32_t nb,
-                                             uint32_t k1, Xyzz<F> *__restrict__ partials,
-                                             Xyzz<F> *__restrict__ buckets, uint32_t stride,
-                                             uint32_t k2, uint32_t q)
+__global__ void __launch_bounds__(128) k_fix_up(const uint32_t *__restrict__ offsets, uint32_t nb, uint32_t kmax,
+                                                 Xyzz<F> *partials, Xyzz<F> *__restrict__ buckets, FixList fix)
 {
-    const uint32_t b = upper_bound_u32(lead_off, nb + 1, q) - 1;
-    const uint32_t j = q - lead_off[b];
-    const Pieces pc = bucket_pieces(offsets, b, k1);
-    const uint32_t off_b = offsets[b];
-    const uint32_t live = (pc.count + stride - 1) / stride;
-    const uint64_t r = uint64_t(j) * k2 * stride;
-    Xyzz<CF<F>> acc = Xyzz<CF<F>>::inf();
-    for (uint32_t m = 0; m < k2; ++m) {
-        const uint64_t idx = r + uint64_t(m) * stride;
-        if (idx >= pc.count) break;
-        acc = xyzz_add(acc, ldx(partials[pc.slot(off_b, k1, uint32_t(idx))]));
+    using C = QF<F>;
+    const uint32_t n = min(*fix.base, fix.cap);
+    const uint32_t k1 = seg_len(offsets[nb], kmax);
+    const uint32_t quads = gridDim.x * blockDim.x / 4;
+    for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) / 4; i < n; i += quads) {
+        const uint2 item = fix.items()[i];
+        const uint32_t b = item.x;
+        uint32_t g = item.y;
+        const uint32_t off_b = offsets[b];
+        const Pieces pc = bucket_pieces(offsets, b, k1);
+        uint64_t stride = 1; // pieces between two inputs of this level
+        for (uint32_t level = 1;; ++level, stride *= kFixGroup) {
+            const uint64_t beg = uint64_t(g) * kFixGroup * stride;
+            C acc = quad_inf<C>();
+            for (uint32_t m = 0; m < kFixGroup; ++m) {
+                const uint64_t idx = beg + m * stride;
+                if (idx >= pc.count) break;
+                acc = quad_add(acc, quad_ld(&partials[pc.slot(off_b, k1, uint32_t(idx))]));
+            }
+            const uint32_t groups = uint32_t((pc.count + kFixGroup * stride - 1) / (kFixGroup * stride));
+            if (groups == 1) {
+                quad_st(&buckets[b], acc);
+                break;
+            }
+            quad_st(&partials[pc.slot(off_b, k1, uint32_t(beg))], acc);
+            g /= kFixGroup;
+            const uint32_t children = min(kFixGroup, groups - g * kFixGroup);
+            if (children > 1) {
+                __threadfence();
+                __syncwarp(quad_mask());
+                uint32_t before = 0;
+                if (quad_role() == 0) {
+                    const uint64_t piece = uint64_t(g) * kFixGroup * kFixGroup * stride + level;
+                    before = atomicAdd(&fix.counters()[pc.slot(off_b, k1, uint32_t(piece))], 1u);
+                }
+                before = __shfl_sync(quad_mask(), before, 0, 4);
+                if (before + 1 != children) break;
+                __threadfence();
+            }
+        }
     }
-    if (live <= k2)
-        buckets[b] = stx(acc);
-    else
-        partials[pc.slot(off_b, k1, uint32_t(r))] = stx(acc);
-}
-
-// Fix-up level: a grid-stride loop over the level's groups (often none).
-template <class F>
-__global__ void __launch_bounds__(128) k_acc_up(const uint32_t *__restrict__ offsets,
-                                                 const uint32_t *__restrict__ lead_off, uint32_t nb,
-                                                 uint32_t k1, Xyzz<F> *__restrict__ partials,
-                                                 Xyzz<F> *__restrict__ buckets, uint32_t stride,
-                                                 uint32_t k2)
-{
-    const uint32_t total = lead_off[nb];
-    for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < total; q += gridDim.x * blockDim.x)
-        acc_up_group(offsets, lead_off, nb, k1, partials, buckets, stride, k2, q);
 }
 
 // --------------------------------------------------------------------------
 // bucket reduction: sum_b b * S_b per set, then + sum_b S_b
 // --------------------------------------------------------------------------
 
-// Buckets per thread (G2: per lane pair) of the first reduction level (log2).
-// The block levels that follow are latency bound (dependent additions), so the
-// first level leaves about 128 x BS items: the next level is then one wave of 128
-// blocks (at most one 256-thread block per SM fits) and a single final block.
-// Measured fastest for G1 (BS 256) at 2^15, 2^16 and 2^19 buckets and G2 (BS 128)
-// at 2^15 and 2^16.
+constexpr int kReduceItems = 64; // items (quads) per block of the block levels
+constexpr int kReduceLog2 = 6;
+
+// Buckets per quad of the first reduction level (log2): about 2^12 quads per set, two
+// thirds of a warp per scheduler, where an addition still runs at its own latency;
+// at most 16 buckets, beyond which more quads share the schedulers.
 // The environment variable NKR_B200_REDUCE_L2 sets it for tuning experiments.
-int first_level_log2(uint32_t m, int log2_bs, int bias)
+int first_level_log2(uint32_t m, int bias)
 {
     static const int forced = [] {
         const char *e = std::getenv("NKR_B200_REDUCE_L2");
@@ -685,7 +551,7 @@ int first_level_log2(uint32_t m, int log2_bs, int bias)
     int lg = 0;
     while ((uint64_t(1) << (lg + 1)) <= m) ++lg;
     if (forced >= 0) return forced < lg ? forced : lg;
-    const int over = lg - (7 + log2_bs);
+    const int over = lg - 12;
     int l2 = (over <= 0 ? 0 : over > 4 ? 4 : over) + bias;
     l2 = l2 < 0 ? 0 : l2;
     return l2 < lg ? l2 : lg;
@@ -694,167 +560,173 @@ int first_level_log2(uint32_t m, int log2_bs, int bias)
 // run += S_b for bucket b: S_b is empty, written whole by the level-1 kernel
 // (one piece) or by the fix-up levels (more than kSmallPieces pieces), or else
 // its few pieces are added straight from the partial slots.
-template <class C, class F>
-__device__ __forceinline__ Xyzz<C> add_bucket_sum(Xyzz<C> run,
-                                                      const uint32_t *__restrict__ offsets,
-                                                      const Xyzz<F> *__restrict__ partials,
-                                                      const Xyzz<F> *__restrict__ buckets, uint32_t b,
-                                                      uint32_t k1)
+template <class F>
+__device__ __forceinline__ QF<F> quad_add_bucket(QF<F> run, const uint32_t *__restrict__ offsets,
+                                                 const Xyzz<F> *partials, const Xyzz<F> *buckets, uint32_t b,
+                                                 uint32_t k1)
 {
     const uint32_t lo = offsets[b], hi = offsets[b + 1];
     if (hi == lo) return run;
     const Pieces pc{lo / k1, (hi - 1) / k1 - lo / k1 + 1};
-    if (pc.count == 1 || pc.count > kSmallPieces) return xyzz_add(run, ldr<C>(buckets[b]));
-    for (uint32_t k = 0; k < pc.count; ++k) run = xyzz_add(run, ldr<C>(partials[pc.slot(lo, k1, k)]));
+    if (pc.count == 1 || pc.count > kSmallPieces) return quad_add(run, quad_ld(&buckets[b]));
+    for (uint32_t k = 0; k < pc.count; ++k) run = quad_add(run, quad_ld(&partials[pc.slot(lo, k1, k)]));
     return run;
 }
 
-// Work-efficient first reduction level: a thread (G2: a lane pair) takes L consecutive buckets
-// and forms T = sum_i i S_i and R = sum_i S_i by running sums (2 additions per
-// bucket), emitting one (A = T, R) item per L buckets with unit L for the block
-// levels that follow.  Bucket sums of few pieces are finished here.
-template <class F, int LANES>
-__global__ void __launch_bounds__(128) k_reduce_first(const uint32_t *__restrict__ offsets,
-                                                       const Xyzz<F> *__restrict__ partials,
-                                                       const Xyzz<F> *__restrict__ buckets,
-                                                       uint64_t items, uint32_t L, uint32_t k1,
+// First reduction level: a quad takes L consecutive buckets and forms
+// T = sum_i i S_i and R = sum_i S_i by running sums (2 additions per bucket), emitting
+// one (A = T, R) item per L buckets with unit L for the block levels that follow.
+// Bucket sums of few pieces are finished here.
+template <class F>
+__global__ void __launch_bounds__(128) k_reduce_first(const uint32_t *__restrict__ offsets, uint32_t nb,
+                                                       const Xyzz<F> *partials, const Xyzz<F> *buckets,
+                                                       uint64_t items, uint32_t L, uint32_t kmax,
                                                        Xyzz<F> *__restrict__ a_out,
                                                        Xyzz<F> *__restrict__ r_out)
 {
-    using C = typename MsmReduceArith<F, LANES>::type;
-    const uint64_t t = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) / LANES; // the lanes' item
+    using C = QF<F>;
+    const uint64_t t = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) / 4;
     if (t * L >= items) return;
+    const uint32_t k1 = seg_len(offsets[nb], kmax);
     const uint64_t base = t * L;
-    Xyzz<C> run = Xyzz<C>::inf(), tri = Xyzz<C>::inf();
+    C run = quad_inf<C>(), tri = quad_inf<C>();
     for (int i = int(L) - 1; i >= 0; --i) {
-        run = add_bucket_sum<C>(run, offsets, partials, buckets, uint32_t(base + i), k1);
-        if (i > 0) tri = xyzz_add(tri, run);
+        run = quad_add_bucket<F>(run, offsets, partials, buckets, uint32_t(base + i), k1);
+        if (i > 0) tri = quad_add(tri, run);
     }
-    if (threadIdx.x % LANES) return;
-    a_out[t] = stx(tri);
-    r_out[t] = stx(run);
+    quad_st(&a_out[t], tri);
+    quad_st(&r_out[t], run);
 }
 
+// A block's points in shared memory, one coordinate per thread: word w of thread j's
+// coordinate at w * BS * 4 + j
+template <class C, int BS>
+struct QuadBuf {
+    uint32_t *s;
+    static constexpr int words = sizeof(C) / 4;
+    __device__ __forceinline__ C ld(int item) const
+    {
+        union {
+            uint32_t w[words];
+            C c;
+        } u;
+        const uint32_t *p = s + item * 4 + quad_role();
+#pragma unroll
+        for (int j = 0; j < words; ++j) u.w[j] = p[j * BS * 4];
+        return u.c;
+    }
+    __device__ __forceinline__ void st(int item, const C &v) const
+    {
+        union U {
+            uint32_t w[words];
+            C c;
+            __device__ U() {}
+        } u;
+        u.c = v;
+        uint32_t *p = s + item * 4 + quad_role();
+#pragma unroll
+        for (int j = 0; j < words; ++j) p[j * BS * 4] = u.w[j];
+    }
+};
+
 // One level of the weighted sum: items carry (A_c, R_c) with
-// S = sum_c (A_c + c U R_c) (unit U = 2^log2_unit; level 0 is A = 0, R = the
-// buckets, U = 1).  A block takes BS consecutive
-// items c (padding with infinity), forms the suffix sums Suf_c = sum_{c' >= c} R_c'
-// with a Hillis-Steele scan in shared memory (log2 BS dependent additions),
-// then sum_c c R_c = sum_{c >= 1} Suf_c and sum_c A_c by two tree sums on
-// disjoint threads, so a level costs about 2 log2(BS) dependent additions
-// instead of 2 BS.  With lane pairs (G2) item c belongs to lanes (2c, 2c + 1)
-// and the even lane stores.
+// S = sum_c (A_c + c U R_c) (unit U = 2^log2_unit).  A block takes BS consecutive
+// items c (padding with infinity), one per quad, forms the suffix sums
+// Suf_c = sum_{c' >= c} R_c' with a Hillis-Steele scan in shared memory (log2 BS dependent
+// additions), then sum_c c R_c = sum_{c >= 1} Suf_c and sum_c A_c by two tree sums on
+// disjoint quads, so a level costs about 2 log2(BS) dependent additions.  BS is 64:
+// two warps per scheduler, beyond which the products of a step queue for the pipe.
 // Output per block: A' = sum A_c + U sum_c c R_c, R' = sum R_c.
-template <class F, int BS, int LANES>
-__global__ void __launch_bounds__(BS * LANES) k_reduce_block(const Xyzz<F> *__restrict__ a_in,
+template <class F, int BS>
+__global__ void __launch_bounds__(BS * 4) k_reduce_block(const Xyzz<F> *__restrict__ a_in,
                                                       const Xyzz<F> *__restrict__ r_in,
                                                       uint32_t m, int log2_unit,
                                                       Xyzz<F> *__restrict__ a_out,
                                                       Xyzz<F> *__restrict__ r_out)
 {
-    using C = typename MsmReduceArith<F, LANES>::type;
-    extern __shared__ uint8_t smem_raw[];
-    Xyzz<C> *buf0 = reinterpret_cast<Xyzz<C> *>(smem_raw);
-    Xyzz<C> *buf1 = buf0 + BS;
+    using C = QF<F>;
+    extern __shared__ uint32_t sm_words[];
+    QuadBuf<C, BS> cur{sm_words}, nxt{sm_words + QuadBuf<C, BS>::words * BS * 4};
     const uint32_t blocks_per_set = (m + BS - 1) / BS;
     const uint32_t set = blockIdx.x / blocks_per_set;
     const uint32_t blk = blockIdx.x % blocks_per_set;
-    const int i = threadIdx.x / LANES;
-    const bool lead = threadIdx.x % LANES == 0;
+    const int i = threadIdx.x / 4;
     const uint64_t idx = uint64_t(blk) * BS + i;
     const bool live = idx < m;
     const uint64_t g = uint64_t(set) * m + idx;
-    Xyzz<C> v = live ? ldr<C>(r_in[g]) : Xyzz<C>::inf();
-    if (lead) buf0[i] = v;
+    C v = live ? quad_ld(&r_in[g]) : quad_inf<C>();
+    cur.st(i, v);
     __syncthreads();
-    Xyzz<C> *cur = buf0, *nxt = buf1;
     for (int d = 1; d < BS; d <<= 1) {
-        if (i + d < BS) v = xyzz_add(v, cur[i + d]);
-        if (lead) nxt[i] = v;
+        if (i + d < BS) v = quad_add(v, cur.ld(i + d));
+        nxt.st(i, v);
         __syncthreads();
-        Xyzz<C> *t = cur;
+        const QuadBuf<C, BS> t = cur;
         cur = nxt;
         nxt = t;
     }
     // v = Suf_i.  R' = Suf_0; weighted part = sum_{i >= 1} Suf_i; A part = sum A_i
-    const Xyzz<C> total = cur[0];
+    nxt.st(i, i >= 1 ? v : quad_inf<C>());
     __syncthreads();
-    if (lead) {
-        buf0[i] = i >= 1 ? v : Xyzz<C>::inf();
-        buf1[i] = (a_in && live) ? ldr<C>(a_in[g]) : Xyzz<C>::inf();
-    }
+    cur.st(i, live ? quad_ld(&a_in[g]) : quad_inf<C>());
     __syncthreads();
-    // the two tree sums run side by side on disjoint lane pairs (first s: weighted
-    // suffix sums, next s: A items), one addition per pair and step; the pair has
-    // read its operands before the even lane overwrites the first (__syncwarp)
+    // the two tree sums side by side on disjoint quads (first s: weighted suffix
+    // sums, next s: A items), one addition per quad and step
     for (int s = BS / 2; s > 0; s >>= 1) {
-        if (i < s) {
-            const Xyzz<C> r = xyzz_add(buf0[i], buf0[i + s]);
-            if constexpr (LANES == 2) __syncwarp(pair_mask());
-            if (lead) buf0[i] = r;
-        } else if (i < 2 * s) {
-            const int j = i - s;
-            const Xyzz<C> r = xyzz_add(buf1[j], buf1[j + s]);
-            if constexpr (LANES == 2) __syncwarp(pair_mask());
-            if (lead) buf1[j] = r;
-        }
+        if (i < s)
+            nxt.st(i, quad_add(nxt.ld(i), nxt.ld(i + s)));
+        else if (i < 2 * s)
+            cur.st(i - s, quad_add(cur.ld(i - s), cur.ld(i)));
         __syncthreads();
     }
     if (i == 0) {
-        Xyzz<C> w = buf0[0];
-        for (int d = 0; d < log2_unit; ++d) w = xyzz_dbl(w);
-        const Xyzz<C> a = xyzz_add(w, buf1[0]);
-        if (lead) {
-            const uint32_t o = set * blocks_per_set + blk;
-            a_out[o] = stx(a);
-            r_out[o] = stx(total);
-        }
+        C w = nxt.ld(0);
+        for (int d = 0; d < log2_unit; ++d) w = quad_dbl(w);
+        const uint32_t o = set * blocks_per_set + blk;
+        quad_st(&a_out[o], quad_add(w, cur.ld(0)));
+        quad_st(&r_out[o], v);
     }
 }
 
 // XYZZ -> libff Jacobian layout without inversion: with Z = ZZ ZZZ,
-// X' = X ZZ ZZZ^2 and Y' = Y ZZ^3 ZZZ^2 represent the same affine point; the
-// coordinates leave the R' domain here (back to the library's R = 2^256).
-template <class C, class F>
-__device__ __forceinline__ void store_jacobian(const Xyzz<C> &p, F *out)
+// X' = X Z ZZZ and Y' = Y Z^2 ZZ represent the same affine point
+template <class F>
+__device__ __forceinline__ void quad_store_jacobian(const QF<F> &v, F *out)
 {
-    if (p.is_inf()) {
-        out[0] = F::zero();
-        out[1] = F::one();
-        out[2] = F::zero();
+    using C = QF<F>;
+    const unsigned role = quad_role();
+    if (quad_is_inf(v)) {
+        if (role < 3) out[role] = role == 1 ? F::one() : F::zero();
         return;
     }
-    const C zzz2 = sqr(p.zzz);
-    const C zz2 = sqr(p.zz);
-    out[0] = msm_out(msm_leave(p.x * (p.zz * zzz2)));
-    out[1] = msm_out(msm_leave(p.y * (zz2 * p.zz * zzz2)));
-    out[2] = msm_out(msm_leave(p.zz * p.zzz));
+    const C zz = quad_get(v, 2), zzz = quad_get(v, 3);
+    const C z = zz * zzz;
+    const C t = select(role == 1, z * zz, zzz);
+    const C u = v * (z * t); // lane 0: X Z ZZZ, lane 1: Y Z^2 ZZ
+    if (role < 3) out[role] = msm_out(role == 2 ? z : u);
 }
 
-// one thread (G2: the lane pair 0, 1); lane 0 stores
-template <class F, int LANES>
-__global__ void k_finalize(const Xyzz<F> *a, const Xyzz<F> *r, int sets, int c, F *out)
-{
-    if (threadIdx.x >= unsigned(LANES) || blockIdx.x != 0) return;
-    using C = typename MsmReduceArith<F, LANES>::type;
-    Xyzz<C> acc = Xyzz<C>::inf();
-    for (int k = sets - 1; k >= 0; --k) {
-        if (k != sets - 1)
-            for (int d = 0; d < c; ++d) acc = xyzz_dbl(acc);
-        acc = xyzz_add(acc, a ? xyzz_add(ldr<C>(a[k]), ldr<C>(r[k])) : ldr<C>(r[k]));
-    }
-    if (threadIdx.x == 0) store_jacobian(acc, out);
-}
-
-// Resident bases enter the R' domain once they are final (x 2^4 mod p per
-// coordinate; the infinity encoding (0, one) maps to (0, one'))
+// The sum of the sets' results, 2^c apart: quad k adds a[k] + r[k], quad 0 runs the Horner
+// chain over them (one set: no chain)
+constexpr int kFinalSets = 64;
 template <class F>
-__global__ void k_bases_to_r260(Affine<F> *__restrict__ pts, uint64_t n)
+__global__ void __launch_bounds__(4 * kFinalSets) k_finalize(const Xyzz<F> *a, const Xyzz<F> *r, int sets, int c,
+                                                              F *out)
 {
-    const uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const Affine<CF<F>> a = lda(pts[i]);
-    pts[i] = {msm_out(msm_enter(a.x)), msm_out(msm_enter(a.y))};
+    using C = QF<F>;
+    extern __shared__ uint32_t sm_words[];
+    const QuadBuf<C, kFinalSets> sum{sm_words};
+    const int i = threadIdx.x / 4;
+    if (i < sets) sum.st(i, quad_add(quad_ld(&a[i]), quad_ld(&r[i])));
+    __syncthreads();
+    if (i > 0) return;
+    C acc = sum.ld(sets - 1);
+    for (int k = sets - 2; k >= 0; --k) {
+        if (!quad_is_inf(acc))
+            for (int d = 0; d < c; ++d) acc = quad_dbl(acc);
+        acc = quad_add(acc, sum.ld(k));
+    }
+    quad_store_jacobian<F>(acc, out);
 }
 
 // --------------------------------------------------------------------------
@@ -928,12 +800,10 @@ __global__ void k_window_chain(const Affine<F> *__restrict__ pts, Xyzz<F> *__res
         for (int k = 1; k < W; ++k) out[uint64_t(k - 1) * m + i] = Xyzz<F>::inf();
         return;
     }
-    const Affine<C> a = lda(s);
-    Xyzz<C> x = xyzz_from_affine_dbl(Affine<C>{msm_enter(a.x), msm_enter(a.y)});
+    Xyzz<C> x = xyzz_from_affine_dbl(lda(s));
     for (int k = 1; k < W; ++k) {
         for (int d = (k == 1 ? 1 : 0); d < c; ++d) x = xyzz_dbl(x);
-        out[uint64_t(k - 1) * m + i] = {msm_out(msm_leave(x.x)), msm_out(msm_leave(x.y)),
-                                        msm_out(msm_leave(x.zz)), msm_out(msm_leave(x.zzz))};
+        out[uint64_t(k - 1) * m + i] = stx(x);
     }
 }
 
@@ -1001,6 +871,21 @@ int build_windows_t(MsmBases &b, cudaStream_t st)
 }
 
 template <class F>
+int launch_level1(uint64_t segs, const uint32_t *offsets, const uint32_t *entries, const Affine<F> *pts, uint32_t nb,
+                  uint32_t kmax, Xyzz<F> *partials, Xyzz<F> *buckets, const DevBuf &fix, cudaStream_t st)
+{
+    if (segs == 0) return NKR_B200_OK;
+    const FixList fl{fix.as<uint32_t>(), fix_cap(segs)};
+    NKR_CUDA(cudaMemsetAsync(fl.base, 0, 4, st));
+    if constexpr (std::is_same<F, Fq>::value)
+        k_acc_l1_g1<<<blocks_for(segs, 128), 128, 0, st>>>(offsets, entries, pts, nb, kmax, partials, buckets, fl);
+    else
+        k_acc_l1_g2<<<blocks_for(segs, 128), 128, 0, st>>>(offsets, entries, pts, nb, kmax, partials, buckets, fl);
+    NKR_CHECK_LAUNCH();
+    return NKR_B200_OK;
+}
+
+template <class F>
 int acc_level1_t(const MsmBases &bs, const MsmSort &s, MsmAcc &a, cudaStream_t st)
 {
     const MsmShape &sh = bs.shape;
@@ -1008,15 +893,8 @@ int acc_level1_t(const MsmBases &bs, const MsmSort &s, MsmAcc &a, cudaStream_t s
     const uint64_t segs = sh.segments_max();
     const uint32_t *offsets = s.offsets.as<uint32_t>();
     if (a.timing) NKR_CUDA(cudaEventRecord(a.ev_acc[0], st));
-    if constexpr (std::is_same<F, Fq>::value)
-        k_acc_l1_g1<<<blocks_for(segs, 128), 128, 0, st>>>(
-            offsets, s.entries.as<uint32_t>(), bs.pts.as<Affine<F>>(), sh.nb, uint32_t(sh.k1),
-            a.partials.as<Xyzz<F>>(), a.buckets.as<Xyzz<F>>());
-    else
-        k_acc_l1_g2<<<blocks_for(segs, 128), 128, 0, st>>>(
-            offsets, s.entries.as<uint32_t>(), bs.pts.as<Affine<F>>(), sh.nb, uint32_t(sh.k1),
-            a.partials.as<Xyzz<F>>(), a.buckets.as<Xyzz<F>>());
-    NKR_CHECK_LAUNCH();
+    NKR_TRY(launch_level1<F>(segs, offsets, s.entries.as<uint32_t>(), bs.pts.as<Affine<F>>(), sh.nb,
+                             uint32_t(sh.k1), a.partials.as<Xyzz<F>>(), a.buckets.as<Xyzz<F>>(), a.fix, st));
     if (a.timing) NKR_CUDA(cudaEventRecord(a.ev_acc[1], st));
     return NKR_B200_OK;
 }
@@ -1037,8 +915,11 @@ int acc_level1_list_t(const MsmAccJob *jobs, int n, void *items_host, void *item
         it.pts = jobs[i].bases->pts.as<Affine<F>>();
         it.partials = jobs[i].acc->partials.as<Xyzz<F>>();
         it.buckets = jobs[i].acc->buckets.as<Xyzz<F>>();
+        it.fix_base = jobs[i].acc->fix.as<uint32_t>();
+        it.fix_capacity = fix_cap(sh.segments_max());
         it.nb = sh.nb;
-        it.k1 = uint32_t(sh.k1);
+        it.kmax = uint32_t(sh.k1);
+        if (sh.segments_max()) NKR_CUDA(cudaMemsetAsync(it.fix_base, 0, 4, st));
         it.first_block = uint32_t(blocks);
         blocks += blocks_for(sh.segments_max(), 128);
         NKR_REQUIRE(blocks < (uint64_t(1) << 31), "batched accumulation too large");
@@ -1054,28 +935,26 @@ int acc_level1_list_t(const MsmAccJob *jobs, int n, void *items_host, void *item
 }
 
 // The reduction levels of an MSM whose buckets are final: first level, block
-// levels, final combination, with LANES lanes per item.
-template <class F, int LANES>
+// levels, final combination.
+template <class F>
 int reduce_run(const MsmBases &bs, const MsmSort &s, MsmAcc &a, void *out_dev, cudaStream_t st)
 {
-    using RA = MsmReduceArith<F, LANES>;
     const MsmShape &sh = bs.shape;
     const uint32_t *offsets = s.offsets.as<uint32_t>();
     const uint32_t sets = sh.folded ? 1u : uint32_t(sh.W);
+    NKR_REQUIRE(sets <= uint32_t(kFinalSets), "%u windows exceed the final combination's %d", sets, kFinalSets);
     uint32_t m = sh.B;
     Xyzz<F> *bufs_a[2] = {a.red_a.as<Xyzz<F>>(), a.red_a2.as<Xyzz<F>>()};
     Xyzz<F> *bufs_r[2] = {a.red_r.as<Xyzz<F>>(), a.red_r2.as<Xyzz<F>>()};
-    constexpr int BS = RA::items;
-    constexpr int kLog2BS = RA::log2_items;
-    const size_t smem = 2 * BS * sizeof(Xyzz<typename RA::type>);
-    NKR_CUDA(cudaFuncSetAttribute(k_reduce_block<F, BS, LANES>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  int(smem)));
+    constexpr int BS = kReduceItems;
+    const size_t smem = 2 * 4 * BS * sizeof(QF<F>);
+    NKR_CUDA(cudaFuncSetAttribute(k_reduce_block<F, BS>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
     // first level: bucket sums (few-piece buckets finished here), L buckets per item
-    const int log2_l = first_level_log2(m, kLog2BS, a.first_level_bias);
+    const int log2_l = first_level_log2(m, a.first_level_bias);
     const uint32_t L = 1u << log2_l;
     const uint64_t items = uint64_t(sets) * m;
-    k_reduce_first<F, LANES><<<blocks_for(LANES * (items / L), 128), 128, 0, st>>>(
-        offsets, a.partials.as<Xyzz<F>>(), a.buckets.as<Xyzz<F>>(), items, L, uint32_t(sh.k1), bufs_a[0],
+    k_reduce_first<F><<<blocks_for(4 * (items / L), 128), 128, 0, st>>>(
+        offsets, sh.nb, a.partials.as<Xyzz<F>>(), a.buckets.as<Xyzz<F>>(), items, L, uint32_t(sh.k1), bufs_a[0],
         bufs_r[0]);
     NKR_CHECK_LAUNCH();
     if (a.timing) NKR_CUDA(cudaEventRecord(a.ev_acc[3], st));
@@ -1086,54 +965,45 @@ int reduce_run(const MsmBases &bs, const MsmSort &s, MsmAcc &a, void *out_dev, c
     int log2_unit = log2_l;
     while (m > 1) {
         const uint32_t per_set = (m + BS - 1) / BS;
-        k_reduce_block<F, BS, LANES><<<sets * per_set, LANES * BS, smem, st>>>(
-            a_in, r_in, m, log2_unit, bufs_a[flip], bufs_r[flip]);
+        k_reduce_block<F, BS><<<sets * per_set, 4 * BS, smem, st>>>(a_in, r_in, m, log2_unit, bufs_a[flip],
+                                                                    bufs_r[flip]);
         NKR_CHECK_LAUNCH();
         a_in = bufs_a[flip];
         r_in = bufs_r[flip];
         flip ^= 1;
         m = per_set;
-        log2_unit += kLog2BS;
+        log2_unit += kReduceLog2;
     }
-    k_finalize<F, LANES><<<1, 32, 0, st>>>(a_in, r_in, int(sets), sh.c, static_cast<F *>(out_dev));
+    // blocks of the sets' quads only (whole warps)
+    k_finalize<F><<<1, sets <= 8 ? 32 : 4 * kFinalSets, 4 * kFinalSets * sizeof(QF<F>), st>>>(
+        a_in, r_in, int(sets), sh.c, static_cast<F *>(out_dev));
     NKR_CHECK_LAUNCH();
     if (a.timing) NKR_CUDA(cudaEventRecord(a.ev_acc[4], st));
     return NKR_B200_OK;
 }
 
-// Fix-up levels of a level-1 accumulation with shape sh (segments, buckets,
-// k1, k2) whose bucket offsets are `offsets`: inputs spaced `stride` pieces
-// apart, groups of k2; one bucket has at most segs + 1 pieces, all buckets at
-// most 2 segs.
+// Fix-up levels of a level-1 accumulation with shape sh (segments, buckets, k1) whose
+// bucket offsets are `offsets`
 template <class F>
-int fixup_levels_t(const MsmShape &sh, const uint32_t *offsets, uint32_t *lead_off, uint32_t *scan_tmp,
-                   Xyzz<F> *partials, Xyzz<F> *buckets, cudaStream_t st)
+int fixup_t(const MsmShape &sh, const uint32_t *offsets, Xyzz<F> *partials, Xyzz<F> *buckets, const DevBuf &fix,
+            cudaStream_t st)
 {
     const uint64_t segs = sh.segments_max();
-    const uint64_t k2 = uint64_t(sh.k2);
-    for (uint64_t stride = 1; stride < segs + 1; stride *= k2) {
-        NKR_TRY(scan_exclusive(LoadLeaders{offsets, uint32_t(sh.k1), uint32_t(stride), uint32_t(k2)},
-                               sh.nb, lead_off, scan_tmp, st));
-        const uint64_t bound = 2 * segs / (stride * k2) + sh.nb + 1;
-        const unsigned grid = std::min<unsigned>(blocks_for(bound, 128), kFixupBlocks);
-        k_acc_up<F><<<grid, 128, 0, st>>>(offsets, lead_off, sh.nb, uint32_t(sh.k1), partials, buckets,
-                                           uint32_t(stride), uint32_t(k2));
-        NKR_CHECK_LAUNCH();
-    }
+    if (segs <= kSmallPieces) return NKR_B200_OK; // no bucket has more pieces than segments
+    const FixList fl{fix.as<uint32_t>(), fix_cap(segs)};
+    const unsigned grid = std::min<unsigned>(blocks_for(4ull * fl.cap, 128), kFixupBlocks);
+    k_fix_up<F><<<grid, 128, 0, st>>>(offsets, sh.nb, uint32_t(sh.k1), partials, buckets, fl);
+    NKR_CHECK_LAUNCH();
     return NKR_B200_OK;
 }
 
 template <class F>
 int acc_tail_t(const MsmBases &bs, const MsmSort &s, MsmAcc &a, void *out_dev, cudaStream_t st)
 {
-    NKR_TRY(fixup_levels_t<F>(bs.shape, s.offsets.as<uint32_t>(), a.lead_off.as<uint32_t>(),
-                              a.scan_tmp.as<uint32_t>(), a.partials.as<Xyzz<F>>(), a.buckets.as<Xyzz<F>>(),
-                              st));
+    NKR_TRY(fixup_t<F>(bs.shape, s.offsets.as<uint32_t>(), a.partials.as<Xyzz<F>>(), a.buckets.as<Xyzz<F>>(), a.fix,
+                       st));
     if (a.timing) NKR_CUDA(cudaEventRecord(a.ev_acc[2], st));
-    // bucket reduction levels (G2 alone: on lane pairs)
-    if constexpr (std::is_same<F, Fq2>::value)
-        if (a.lane_pairs) return reduce_run<F, 2>(bs, s, a, out_dev, st);
-    return reduce_run<F, 1>(bs, s, a, out_dev, st);
+    return reduce_run<F>(bs, s, a, out_dev, st);
 }
 
 template <class F>
@@ -1147,21 +1017,16 @@ template <class F>
 int acc_alloc_t(MsmAcc &a, const MsmShape &sh)
 {
     const uint32_t sets = sh.folded ? 1u : uint32_t(sh.W);
-    // first reduction level output: one item per L buckets (L as in acc_run_t)
-    // items per block of the reduction levels (the same for one and two lanes per item)
-    constexpr int kLog2BS = MsmReduceArith<F, 1>::log2_items;
-    static_assert(MsmReduceArith<F, 1>::log2_items == MsmReduceArith<F, 2>::log2_items || sizeof(F) == sizeof(Fq),
-                  "G2 reduction buffers are sized for one block shape");
-    const uint64_t red = uint64_t(sets) * (sh.B >> first_level_log2(sh.B, kLog2BS, a.first_level_bias)) + 1;
+    // first reduction level output: one item per L buckets
+    const uint64_t red = uint64_t(sets) * (sh.B >> first_level_log2(sh.B, a.first_level_bias)) + 1;
     NKR_TRY(a.partials.alloc(2 * std::max<uint64_t>(sh.segments_max(), 1) * sizeof(Xyzz<F>),
                              "msm partial sums"));
     NKR_TRY(a.buckets.alloc(uint64_t(sh.nb) * sizeof(Xyzz<F>), "msm buckets"));
-    NKR_TRY(a.lead_off.alloc((sh.nb + 1) * 4ull, "msm fix-up offsets"));
+    NKR_TRY(a.fix.alloc(fix_bytes(sh.segments_max()), "msm fix-up list"));
     NKR_TRY(a.red_a.alloc(red * sizeof(Xyzz<F>), "msm reduction"));
     NKR_TRY(a.red_r.alloc(red * sizeof(Xyzz<F>), "msm reduction"));
     NKR_TRY(a.red_a2.alloc(red * sizeof(Xyzz<F>), "msm reduction"));
     NKR_TRY(a.red_r2.alloc(red * sizeof(Xyzz<F>), "msm reduction"));
-    NKR_TRY(a.scan_tmp.alloc(scan_scratch_words(sh.nb) * 4, "msm scan scratch"));
     NKR_TRY(a.result.alloc(192, "msm result"));
     return NKR_B200_OK;
 }
@@ -1271,52 +1136,41 @@ __global__ void k_cls_scatter(const uint32_t *__restrict__ class_of, const uint3
     entries[base + uint32_t(__popc(peers & ((1u << lane) - 1u)))] = uint32_t(i);
 }
 
-// a class sum as an affine base of the small MSM (storage form of the group's
-// MSM buffers: G1 in the R' domain; infinity as (0, one))
-__device__ __forceinline__ Affine<Fq> class_affine(const Xyzz<Fq52L> &s)
-{
-    if (s.is_inf()) return {from52(Fq52::zero()), from52(Fq52::one())};
-    const Affine<Fq52> a = xyzz_to_affine(Xyzz<Fq52>{s.x.canon(), s.y.canon(), s.zz.canon(), s.zzz.canon()});
-    return {from52(a.x), from52(a.y)};
-}
-__device__ __forceinline__ Affine<Fq2> class_affine(const Xyzz<Fq2> &s) { return xyzz_to_affine(s); }
-
-// S_c for every class: its pieces (level-1 runs and fix-up sums) added up and
-// normalised with one inversion per class
+// S_c for every class: its pieces (level-1 runs and fix-up sums) added up by a quad and
+// normalised with one inversion per class (the quad's lanes run it alike)
 template <class F>
 __global__ void __launch_bounds__(128) k_cls_finish(const uint32_t *__restrict__ offsets,
-                                                     const Xyzz<F> *__restrict__ partials,
-                                                     const Xyzz<F> *__restrict__ buckets, uint32_t k1,
+                                                     const Xyzz<F> *partials, const Xyzz<F> *buckets, uint32_t kmax,
                                                      uint32_t nb, Affine<F> *__restrict__ sums)
 {
-    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
+    using C = QF<F>;
+    const uint32_t c = (blockIdx.x * blockDim.x + threadIdx.x) / 4;
     if (c >= nb) return;
-    using C = CF<F>;
-    sums[c] = class_affine(add_bucket_sum<C>(Xyzz<C>::inf(), offsets, partials, buckets, c, k1));
+    const unsigned role = quad_role();
+    const C v = quad_add_bucket<F>(quad_inf<C>(), offsets, partials, buckets, c, seg_len(offsets[nb], kmax));
+    F *out = &sums[c].x;
+    if (quad_is_inf(v)) {
+        if (role < 2) out[role] = role ? F::one() : F::zero();
+        return;
+    }
+    const C zz = quad_get(v, 2), zzz = quad_get(v, 3);
+    const C t = C(inverse(msm_out(zz * zzz)));           // 1 / (ZZ ZZZ)
+    const C r = v * (t * select(role == 0, zzz, zz));    // lane 0: X / ZZ, lane 1: Y / ZZZ
+    if (role < 2) out[role] = msm_out(r);
 }
 
-// acc += add for two libff-Jacobian points (X, Y, Z; Z = 0 is infinity) in the
-// library's Montgomery domain
+// acc += add for two libff-Jacobian points (X, Y, Z; Z = 0 is infinity)
 template <class F>
 __global__ void k_result_add(F *acc, const F *add)
 {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    auto xyzz = [](const F *p) {
-        if (p[2].is_zero()) return Xyzz<F>::inf();
-        const F zz = sqr(p[2]);
-        return Xyzz<F>{p[0], p[1], zz, zz * p[2]};
+    if (threadIdx.x >= 4 || blockIdx.x != 0) return;
+    using C = QF<F>;
+    const unsigned role = quad_role();
+    auto xyzz = [&](const F *p) {
+        const C z = C(p[2]), zz = z * z, zzz = zz * z;
+        return role < 2 ? C(p[role]) : role == 2 ? zz : zzz;
     };
-    const Xyzz<F> s = xyzz_add(xyzz(acc), xyzz(add));
-    if (s.is_inf()) {
-        acc[0] = F::zero();
-        acc[1] = F::one();
-        acc[2] = F::zero();
-        return;
-    }
-    const F zzz2 = sqr(s.zzz), zz2 = sqr(s.zz);
-    acc[0] = s.x * (s.zz * zzz2);
-    acc[1] = s.y * (zz2 * s.zz * zzz2);
-    acc[2] = s.zz * s.zzz;
+    quad_store_jacobian<F>(quad_add(xyzz(acc), xyzz(add)), acc);
 }
 
 // G2's MSM over its class values uses the twist Frobenius psi(x, y) =
@@ -1381,8 +1235,7 @@ int class_acc_alloc_t(MsmClassAcc &a, uint64_t n)
     const uint64_t segs = std::max<uint64_t>(a.seg.segments_max(), 1);
     NKR_TRY(a.partials.alloc(2 * segs * sizeof(Xyzz<F>), "class partial sums"));
     NKR_TRY(a.buckets.alloc(uint64_t(kClassMax) * sizeof(Xyzz<F>), "class sums"));
-    NKR_TRY(a.lead_off.alloc((kClassMax + 1) * 4ull, "class fix-up offsets"));
-    NKR_TRY(a.scan_tmp.alloc(scan_scratch_words(kClassMax) * 4, "class scan scratch"));
+    NKR_TRY(a.fix.alloc(fix_bytes(segs), "class fix-up list"));
     return NKR_B200_OK;
 }
 
@@ -1391,20 +1244,10 @@ int class_acc_issue_t(const MsmBases &b, const MsmClassSort &cs, MsmClassAcc &a,
 {
     const uint64_t segs = a.seg.segments_max();
     const uint32_t *offsets = cs.offsets.as<uint32_t>();
-    if (segs) {
-        if constexpr (std::is_same<F, Fq>::value)
-            k_acc_l1_g1<<<blocks_for(segs, 128), 128, 0, st>>>(
-                offsets, cs.entries.as<uint32_t>(), b.pts.as<Affine<F>>(), kClassMax, uint32_t(a.seg.k1),
-                a.partials.as<Xyzz<F>>(), a.buckets.as<Xyzz<F>>());
-        else
-            k_acc_l1_g2<<<blocks_for(segs, 128), 128, 0, st>>>(
-                offsets, cs.entries.as<uint32_t>(), b.pts.as<Affine<F>>(), kClassMax, uint32_t(a.seg.k1),
-                a.partials.as<Xyzz<F>>(), a.buckets.as<Xyzz<F>>());
-        NKR_CHECK_LAUNCH();
-    }
-    NKR_TRY(fixup_levels_t<F>(a.seg, offsets, a.lead_off.as<uint32_t>(), a.scan_tmp.as<uint32_t>(),
-                              a.partials.as<Xyzz<F>>(), a.buckets.as<Xyzz<F>>(), st));
-    k_cls_finish<F><<<blocks_for(kClassMax, 128), 128, 0, st>>>(
+    NKR_TRY(launch_level1<F>(segs, offsets, cs.entries.as<uint32_t>(), b.pts.as<Affine<F>>(), kClassMax,
+                             uint32_t(a.seg.k1), a.partials.as<Xyzz<F>>(), a.buckets.as<Xyzz<F>>(), a.fix, st));
+    NKR_TRY(fixup_t<F>(a.seg, offsets, a.partials.as<Xyzz<F>>(), a.buckets.as<Xyzz<F>>(), a.fix, st));
+    k_cls_finish<F><<<blocks_for(4ull * kClassMax, 128), 128, 0, st>>>(
         offsets, a.partials.as<Xyzz<F>>(), a.buckets.as<Xyzz<F>>(), uint32_t(a.seg.k1), kClassMax,
         a.small.pts.as<Affine<F>>());
     NKR_CHECK_LAUNCH();
@@ -1493,12 +1336,6 @@ int msm_bases_build(MsmBases &b, int group, const void *jac, bool jac_on_device,
         NKR_CUDA(cudaStreamSynchronize(st));
     }
     if (folded) NKR_TRY(group == 1 ? build_windows_t<Fq>(b, st) : build_windows_t<Fq2>(b, st));
-    const uint64_t total = n * copies;
-    if (group == 1) { // G2 computes in the library's own domain
-        k_bases_to_r260<Fq><<<blocks_for(total, 128), 128, 0, st>>>(b.pts.as<G1Affine>(), total);
-        NKR_CHECK_LAUNCH();
-    }
-
     NKR_CUDA(cudaStreamSynchronize(st));
     return NKR_B200_OK;
 }
@@ -1711,9 +1548,6 @@ int msm_class_acc_alloc(MsmClassAcc &a, int group, uint64_t n)
         NKR_TRY(a.split.alloc(pts * sizeof(Fr), "class value halves"));
     }
     NKR_TRY(a.small.pts.alloc(pts * (group == 1 ? sizeof(G1Affine) : sizeof(G2Affine)), "class sums (affine)"));
-    // the MSM over the class values ends with a Horner chain of ~250 doublings;
-    // G2 runs its reduction levels on lane pairs (half the chain's latency)
-    a.small_s.acc.lane_pairs = group == 2;
     NKR_TRY(msm_scratch_alloc(a.small_s, group, a.small.shape));
     NKR_TRY(a.out.alloc(group == 1 ? 96 : 192, "class MSM result"));
     return NKR_B200_OK;

@@ -18,13 +18,13 @@
 //     [t K1, (t+1) K1) into XYZZ accumulators (mixed add 8M + 2S, with the
 //     doubling branch), one run per bucket it crosses, so all lanes do equal
 //     work whatever the bucket sizes.  A bucket spread over several segments
-//     leaves one partial per segment and is finished by fix-up levels of fan-in
-//     K2: each level scans, per bucket, how many groups of K2 pieces remain and
-//     gives every group its own thread, so a bucket holding a large share of all
-//     points (repeated or small scalars) costs O(log n) sequential additions.
-//  3. bucket reduction: sum_b (b + 1) S_b in levels of 256 (G1) / 128 (G2)
-//     items per block: a shared-memory suffix scan and tree sums make a level
-//     about 2 log2(block) dependent additions deep.
+//     leaves one partial per segment; a bucket of many pieces is finished by fix-up
+//     levels of fan-in 16, so one holding a large share of all points (repeated or
+//     small scalars) costs O(log n) sequential additions.
+//  3. bucket reduction: sum_b (b + 1) S_b in levels of 64 items per block: a
+//     shared-memory suffix scan and tree sums make a level about 2 log2(block)
+//     dependent additions deep.  From the fix-up levels on four lanes hold a point
+//     and share every addition (quad.cuh).
 //  4. windows: with resident "folded" bases the W windows share one bucket set
 //     because the bases hold the copies 2^(c k) P_i (built once at prepare; HBM
 //     is large); otherwise each window has its own set and a Horner pass
@@ -48,6 +48,19 @@
 
 namespace nkr {
 
+// Entries per level-1 segment (mixed additions per thread) of an MSM of `total` entries:
+// enough segments for one and a half warps per scheduler (148 x 4 x 48 threads), where an
+// addition still runs at its own latency, within kSegMin..kmax entries.  The count is
+// known on the device only (zero digits and class members have no entry), so every
+// kernel that needs the length computes it from the sort's total.
+constexpr uint32_t kSegMin = 4;
+constexpr uint32_t kSegSpread = 148 * 4 * 48;
+__host__ __device__ __forceinline__ uint32_t seg_len(uint32_t total, uint32_t kmax)
+{
+    const uint32_t k = (total + kSegSpread - 1) / kSegSpread;
+    return k < kSegMin ? kSegMin : k > kmax ? kmax : k;
+}
+
 struct MsmShape {
     uint64_t n = 0; // points
     int c = 0;      // window bits
@@ -55,14 +68,15 @@ struct MsmShape {
     bool folded = false;
     uint32_t B = 0;  // buckets per set: 2^(c-1)
     uint32_t nb = 0; // total buckets: folded ? B : W * B
-    // entries per level-1 segment (mixed additions per thread).  Measured slower
-    // at 2^16 points: 8 or 16 (level 1 shorter, fix-ups and the first reduction
-    // level longer); at 2^20: 32-48 sized to whole waves of the kernel (prove
-    // 18.60 -> 18.79 ms)
-    int k1 = 32;
-    int k2 = 16;     // fan-in of the fix-up levels (8 and 4 measured no faster in a prove)
+    int k1 = 32;     // most entries per level-1 segment (seg_len)
     uint64_t entries_max() const { return uint64_t(W) * n; }
-    uint64_t segments_max() const { return (entries_max() + k1 - 1) / k1; }
+    // most segments over all entry counts up to entries_max
+    uint64_t segments_max() const
+    {
+        const uint64_t e = entries_max(), fine = (e + kSegMin - 1) / kSegMin, coarse = (e + k1 - 1) / k1;
+        const uint64_t spread = fine < kSegSpread ? fine : kSegSpread;
+        return coarse > spread ? coarse : spread;
+    }
     bool same_sort(const MsmShape &o) const
     {
         return n == o.n && c == o.c && W == o.W && folded == o.folded && k1 == o.k1;
@@ -83,7 +97,7 @@ struct MsmSort {
 
 // Accumulation state of one MSM (partials, buckets, reduction levels, result).
 struct MsmAcc {
-    DevBuf partials, buckets, lead_off, red_a, red_r, red_a2, red_r2, scan_tmp, result;
+    DevBuf partials, buckets, fix, red_a, red_r, red_a2, red_r2, result;
     // record events at the phase boundaries: before and after the level-1
     // accumulation kernel, after the fix-up levels, after the first reduction
     // level, after the last reduction level and the final combination
@@ -92,13 +106,10 @@ struct MsmAcc {
     // added to the first reduction level's log2 buckets per thread (set before
     // msm_acc_alloc): larger levels do less work in more dependent steps
     int first_level_bias = 0;
-    // G2 reduction levels on lane pairs (two lanes per item): shorter for an MSM
-    // alone, but inside a prove the wider blocks crowd out the other MSMs' work
-    bool lane_pairs = false;
     size_t device_bytes() const
     {
-        return partials.bytes + buckets.bytes + lead_off.bytes + red_a.bytes + red_r.bytes +
-               red_a2.bytes + red_r2.bytes + scan_tmp.bytes + result.bytes;
+        return partials.bytes + buckets.bytes + fix.bytes + red_a.bytes + red_r.bytes + red_a2.bytes +
+               red_r2.bytes + result.bytes;
     }
 };
 
@@ -228,14 +239,14 @@ int msm_class_sort_run(MsmClassSort &s, const MsmDedup &d, const uint32_t *gathe
 // class values.
 struct MsmClassAcc {
     MsmShape seg;      // n = the support's points, nb = kClassMax classes, k1, k2
-    DevBuf partials, buckets, lead_off, scan_tmp;
+    DevBuf partials, buckets, fix;
     MsmBases small;    // the class sums (affine; G2: and their psi images), non-folded
     MsmScratch small_s;
     DevBuf split;      // G2: the class values as k0 + k1 lambda (msm.cu)
     DevBuf out;        // sum_c v_c S_c, libff Jacobian layout
     size_t device_bytes() const
     {
-        return partials.bytes + buckets.bytes + lead_off.bytes + scan_tmp.bytes + small.device_bytes() +
+        return partials.bytes + buckets.bytes + fix.bytes + small.device_bytes() +
                small_s.device_bytes() + split.bytes + out.bytes;
     }
 };

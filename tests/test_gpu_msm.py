@@ -48,6 +48,21 @@ def test_msm_uniform(ctx, orc, rng, group, n, folded):
     _check(ctx, orc, group, aff, sc, folded)
 
 
+@pytest.mark.parametrize("group", [1, 2])
+@pytest.mark.parametrize("pieces", [4, 5, 16, 17, 65, 257, 1025])
+def test_msm_large_buckets_over_fixup_levels(ctx, orc, rng, group, pieces):
+    """One bucket of exactly `pieces` level-1 pieces (segments of 4 entries at these sizes),
+    around each power of the fix-up fan-in 4, with a second bucket of one point in front and
+    behind so that its segments are ragged."""
+    n = 4 * pieces
+    aff = _points(orc, group, n, rng, distinct=min(n, 37))
+    sc = np.tile(O.fr_mont(2), (n, 1))
+    _check(ctx, orc, group, aff, sc, True)            # aligned with the segments
+    sc[rng.integers(0, n)] = O.fr_mont(1)
+    sc[rng.integers(0, n)] = O.fr_mont(3)
+    _check(ctx, orc, group, aff, sc, True)
+
+
 @pytest.mark.parametrize("folded", [False, True])
 @pytest.mark.parametrize("group", [1, 2])
 def test_msm_edge_cases(ctx, orc, rng, group, folded):
