@@ -381,6 +381,38 @@ __device__ __forceinline__ void add_words_carry(uint32_t *r, const uint32_t *x, 
           "r"(y[0]), "r"(y[1]), "r"(y[2]), "r"(y[3]), "r"(y[4]), "r"(y[5]), "r"(y[6]), "r"(y[7]));
 }
 
+// r = x - y on 16 words (no borrow out); r may be x
+__device__ __forceinline__ void sub_words16(uint32_t *r, const uint32_t *x, const uint32_t *y)
+{
+    uint32_t br;
+    asm("sub.cc.u32  %0, %9,  %17;\n\t"
+        "subc.cc.u32 %1, %10, %18;\n\t"
+        "subc.cc.u32 %2, %11, %19;\n\t"
+        "subc.cc.u32 %3, %12, %20;\n\t"
+        "subc.cc.u32 %4, %13, %21;\n\t"
+        "subc.cc.u32 %5, %14, %22;\n\t"
+        "subc.cc.u32 %6, %15, %23;\n\t"
+        "subc.cc.u32 %7, %16, %24;\n\t"
+        "subc.u32    %8, 0, 0;"
+        : "=&r"(r[0]), "=&r"(r[1]), "=&r"(r[2]), "=&r"(r[3]), "=&r"(r[4]), "=&r"(r[5]), "=&r"(r[6]),
+          "=&r"(r[7]), "=&r"(br)
+        : "r"(x[0]), "r"(x[1]), "r"(x[2]), "r"(x[3]), "r"(x[4]), "r"(x[5]), "r"(x[6]), "r"(x[7]),
+          "r"(y[0]), "r"(y[1]), "r"(y[2]), "r"(y[3]), "r"(y[4]), "r"(y[5]), "r"(y[6]), "r"(y[7]));
+    asm("sub.cc.u32  %8, 0,   %8;\n\t" // br is all ones on borrow: borrows again
+        "subc.cc.u32 %0, %9,  %17;\n\t"
+        "subc.cc.u32 %1, %10, %18;\n\t"
+        "subc.cc.u32 %2, %11, %19;\n\t"
+        "subc.cc.u32 %3, %12, %20;\n\t"
+        "subc.cc.u32 %4, %13, %21;\n\t"
+        "subc.cc.u32 %5, %14, %22;\n\t"
+        "subc.cc.u32 %6, %15, %23;\n\t"
+        "subc.u32    %7, %16, %24;"
+        : "=&r"(r[8]), "=&r"(r[9]), "=&r"(r[10]), "=&r"(r[11]), "=&r"(r[12]), "=&r"(r[13]), "=&r"(r[14]),
+          "=&r"(r[15]), "+r"(br)
+        : "r"(x[8]), "r"(x[9]), "r"(x[10]), "r"(x[11]), "r"(x[12]), "r"(x[13]), "r"(x[14]), "r"(x[15]),
+          "r"(y[8]), "r"(y[9]), "r"(y[10]), "r"(y[11]), "r"(y[12]), "r"(y[13]), "r"(y[14]), "r"(y[15]));
+}
+
 // E[0..8], O[0..7] += m p with m = E[0] (-p^-1): word offset 0 becomes zero
 template <class P>
 __device__ __forceinline__ void eo_reduce_row(uint32_t *e, uint32_t *o)
@@ -655,10 +687,8 @@ __device__ __forceinline__ void mul_wide(const uint32_t *a, const uint32_t *b, u
     for (int j = 0; j < 7; ++j) t[9 + j] = hi[j];
 }
 
-// Montgomery reduction T R^-1 mod p of a 512-bit T < p R (R = 2^256): the low half is
-// reduced as in mont_mul (the result is at most p) and added to the high half,
-// below 2p before the final conditional subtraction.
-__device__ __forceinline__ Fq redc_wide(const uint32_t *t)
+// r = t[0..7] R^-1 mod p (R = 2^256), at most p: the rows of mont_mul without a product
+__device__ __forceinline__ void redc_low(const uint32_t *t, uint32_t *r)
 {
     uint32_t e[9], o[8];
 #pragma unroll
@@ -682,9 +712,16 @@ __device__ __forceinline__ Fq redc_wide(const uint32_t *t)
 #pragma unroll
         for (int j = 0; j < 8; ++j) o[j] = no[j];
     }
+    add_words(r, e + 1, o);
+}
+
+// Montgomery reduction T R^-1 mod p of a 512-bit T < p R: the low half's reduction and the
+// high half, below 2p before the conditional subtraction
+__device__ __forceinline__ Fq redc_wide(const uint32_t *t)
+{
     Fq r;
     uint32_t lo[8];
-    add_words(lo, e + 1, o);
+    redc_low(t, lo);
     add_words(r.v, lo, t + 8);
     reduce_once<FqParams>(r.v);
     return r;

@@ -13,7 +13,8 @@
 // computed in affine twist coordinates: for slope lam' on the twist the line
 // at P = (xP, yP) is yP - lam' xP w + (lam' xT - yT) v w (its vertical-line and
 // projective-scale factors lie in proper subfields and vanish in the final
-// exponentiation, so the value after it equals libff's); a per-call point runs
+// exponentiation, so the value after it equals libff's); here are the lines of a
+// key's fixed points, while a per-call point (pairing_lanes.cuh) runs
 // in homogeneous coordinates with Fq2-scaled lines (no inversion per step).
 //
 // Final exponentiation: f^((q^6 - 1)(q^2 + 1) k (q^4 - q^2 + 1)/r) with
@@ -25,19 +26,9 @@
 
 #include "curve.cuh"
 
-// The Fq12-level operations are compiled out of line: inlined, one verification
-// is a single function of several hundred thousand instructions (ptxas runs for
-// minutes and the frame spills kilobytes); out of line, each body exists once.
-#define NKR_PAIR_FN inline __noinline__
-
 namespace nkr {
 
-struct Fq6 {
-    Fq2 c0, c1, c2;
-};
-struct Fq12 {
-    Fq6 c0, c1;
-};
+constexpr size_t kFq12Bytes = 12 * sizeof(Fq); // a GT value in memory (libff alt_bn128_Fq12)
 
 // ---------------------------------------------------------------------------
 // Fq2 helpers
@@ -51,93 +42,6 @@ __device__ __forceinline__ Fq2 mul_xi(const Fq2 &a)
 }
 __device__ __forceinline__ Fq2 mul_fq(const Fq2 &a, const Fq &s) { return {a.c0 * s, a.c1 * s}; }
 __device__ __forceinline__ Fq2 conj(const Fq2 &a) { return {a.c0, neg(a.c1)}; }
-
-// ---------------------------------------------------------------------------
-// Fq6
-// ---------------------------------------------------------------------------
-
-__device__ __forceinline__ Fq6 fq6_zero() { return {Fq2::zero(), Fq2::zero(), Fq2::zero()}; }
-__device__ __forceinline__ Fq6 operator+(const Fq6 &a, const Fq6 &b)
-{
-    return {a.c0 + b.c0, a.c1 + b.c1, a.c2 + b.c2};
-}
-__device__ __forceinline__ Fq6 operator-(const Fq6 &a, const Fq6 &b)
-{
-    return {a.c0 - b.c0, a.c1 - b.c1, a.c2 - b.c2};
-}
-__device__ __forceinline__ Fq6 neg(const Fq6 &a) { return {neg(a.c0), neg(a.c1), neg(a.c2)}; }
-// a v
-__device__ __forceinline__ Fq6 mul_v(const Fq6 &a) { return {mul_xi(a.c2), a.c0, a.c1}; }
-
-// Karatsuba: 6 Fq2 products
-__device__ inline Fq6 operator*(const Fq6 &a, const Fq6 &b)
-{
-    const Fq2 t0 = a.c0 * b.c0, t1 = a.c1 * b.c1, t2 = a.c2 * b.c2;
-    return {t0 + mul_xi((a.c1 + a.c2) * (b.c1 + b.c2) - t1 - t2),
-            (a.c0 + a.c1) * (b.c0 + b.c1) - t0 - t1 + mul_xi(t2),
-            (a.c0 + a.c2) * (b.c0 + b.c2) - t0 - t2 + t1};
-}
-
-__device__ inline Fq6 inverse(const Fq6 &a)
-{
-    const Fq2 t0 = sqr(a.c0) - mul_xi(a.c1 * a.c2);
-    const Fq2 t1 = mul_xi(sqr(a.c2)) - a.c0 * a.c1;
-    const Fq2 t2 = sqr(a.c1) - a.c0 * a.c2;
-    const Fq2 d = a.c0 * t0 + mul_xi(a.c2 * t1 + a.c1 * t2);
-    const Fq2 di = inverse(d);
-    return {t0 * di, t1 * di, t2 * di};
-}
-
-// ---------------------------------------------------------------------------
-// Fq12
-// ---------------------------------------------------------------------------
-
-__device__ __forceinline__ Fq12 fq12_one() { return {{Fq2::one(), Fq2::zero(), Fq2::zero()}, fq6_zero()}; }
-
-__device__ NKR_PAIR_FN Fq12 operator*(const Fq12 &a, const Fq12 &b)
-{
-    const Fq6 t0 = a.c0 * b.c0, t1 = a.c1 * b.c1;
-    return {t0 + mul_v(t1), (a.c0 + a.c1) * (b.c0 + b.c1) - t0 - t1};
-}
-
-// (a0 + a1 w)^2 = (a0 + a1)(a0 + v a1) - t - v t + 2 t w, t = a0 a1
-__device__ NKR_PAIR_FN Fq12 sqr(const Fq12 &a)
-{
-    const Fq6 t = a.c0 * a.c1;
-    return {(a.c0 + a.c1) * (a.c0 + mul_v(a.c1)) - t - mul_v(t), t + t};
-}
-
-__device__ __forceinline__ Fq12 conj(const Fq12 &a) { return {a.c0, neg(a.c1)}; }
-
-__device__ NKR_PAIR_FN Fq12 inverse(const Fq12 &a)
-{
-    const Fq6 t = inverse(a.c0 * a.c0 - mul_v(a.c1 * a.c1));
-    return {a.c0 * t, neg(a.c1 * t)};
-}
-
-__device__ __forceinline__ bool operator==(const Fq12 &a, const Fq12 &b)
-{
-    return a.c0.c0 == b.c0.c0 && a.c0.c1 == b.c0.c1 && a.c0.c2 == b.c0.c2 && a.c1.c0 == b.c1.c0 &&
-           a.c1.c1 == b.c1.c1 && a.c1.c2 == b.c1.c2;
-}
-
-// f times the line yP + a w + b v w (a = -lam xP, b = lam xT - yT):
-// (f0 + f1 w)(L0 + L1 w) = (f0 L0 + v f1 L1) + (f0 L1 + f1 L0) w with L0 = yP,
-// L1 = a + b v
-__device__ __forceinline__ Fq6 mul_by_ab(const Fq6 &f, const Fq2 &a, const Fq2 &b)
-{
-    // (f0 + f1 v + f2 v^2)(a + b v)
-    return {f.c0 * a + mul_xi(f.c2 * b), f.c0 * b + f.c1 * a, f.c1 * b + f.c2 * a};
-}
-__device__ __forceinline__ Fq6 mul_by_fq(const Fq6 &f, const Fq &s)
-{
-    return {mul_fq(f.c0, s), mul_fq(f.c1, s), mul_fq(f.c2, s)};
-}
-__device__ NKR_PAIR_FN Fq12 mul_by_line(const Fq12 &f, const Fq &yP, const Fq2 &a, const Fq2 &b)
-{
-    return {mul_by_fq(f.c0, yP) + mul_v(mul_by_ab(f.c1, a, b)),
-            mul_by_ab(f.c0, a, b) + mul_by_fq(f.c1, yP)};
-}
 
 // ---------------------------------------------------------------------------
 // constants
@@ -217,44 +121,8 @@ __device__ __forceinline__ Fq2 frob_coeff(const Fq2 &a, int k, int m)
     return m ? b * frob_gamma(k, m) : b;
 }
 
-__device__ NKR_PAIR_FN Fq12 frobenius(const Fq12 &x, int k)
-{
-    return {{frob_coeff(x.c0.c0, k, 0), frob_coeff(x.c0.c1, k, 2), frob_coeff(x.c0.c2, k, 4)},
-            {frob_coeff(x.c1.c0, k, 1), frob_coeff(x.c1.c1, k, 3), frob_coeff(x.c1.c2, k, 5)}};
-}
-
-// x^(-z) for x in the cyclotomic subgroup (inverse = conjugate), z = 0x44e992b44a6909f1
+// the curve parameter z
 constexpr uint64_t kZ = 0x44e992b44a6909f1ull;
-__device__ NKR_PAIR_FN Fq12 exp_by_neg_z(const Fq12 &x)
-{
-    Fq12 r = x;
-    for (int b = 61; b >= 0; --b) { // bit 62, the top one, is r = x
-        r = sqr(r);
-        if ((kZ >> b) & 1ull) r = r * x;
-    }
-    return conj(r);
-}
-
-// f^((q^6 - 1)(q^2 + 1)) (the easy part), then libff's last chunk
-// (alt_bn128_pairing.cpp:152-224, Fuentes-Castaneda et al.): the same addition
-// chain, so the result is libff's GT value: elt^(2z(6z^2 + 3z + 1)(q^4 - q^2 + 1)/r)
-__device__ NKR_PAIR_FN Fq12 final_exponentiation(const Fq12 &f)
-{
-    const Fq12 c = conj(f) * inverse(f);
-    const Fq12 elt = frobenius(c, 2) * c;
-    const Fq12 A = exp_by_neg_z(elt);
-    const Fq12 B = sqr(A);
-    const Fq12 C = sqr(B);
-    const Fq12 D = C * B;
-    const Fq12 E = exp_by_neg_z(D);
-    const Fq12 F = sqr(E);
-    const Fq12 G = exp_by_neg_z(F);
-    const Fq12 K = conj(G) * E * conj(D); // 12z^3 + 6z^2 + 6z
-    const Fq12 L = K * B;                 // 12z^3 + 6z^2 + 4z
-    const Fq12 N = K * E * elt;           // 12z^3 + 12z^2 + 6z + 1
-    const Fq12 R = frobenius(K, 2) * (frobenius(L, 1) * N);
-    return frobenius(conj(elt) * L, 3) * R;
-}
 
 // ---------------------------------------------------------------------------
 // Miller loop pieces
@@ -311,64 +179,6 @@ __device__ inline void ate_lines(const Affine<Fq2> &q, AteLine *out)
     out[s++] = ate_add(t, twist_frobenius(q));
     Affine<Fq2> t2 = t;
     out[s++] = ate_add(t2, twist_neg_frobenius2(q));
-}
-
-__device__ __forceinline__ Fq12 apply_line(const Fq12 &f, const AteLine &l, const Affine<Fq> &p)
-{
-    return mul_by_line(f, p.y, neg(mul_fq(l.lam, p.x)), l.c);
-}
-
-// The Miller loop of a point Q that changes per call (a proof's B) runs T in
-// homogeneous coordinates (x = X/Z, y = Y/Z) so that no step inverts.  Its lines
-// are the affine ones times an Fq2 factor (2YZ^2 for a doubling, xQ Z - X for an
-// addition), which the final exponentiation removes: line = c0 + a w + b v w,
-// c0 already multiplied by yP.
-struct G2Proj {
-    Fq2 x, y, z;
-};
-struct ProjLine {
-    Fq2 c0, a, b;
-};
-
-// tangent at T, T <- 2T: with A = 3X^2, B = 2YZ (slope A/B),
-// 2T = ((A^2 Z - 2X B^2) B, A (3X B^2 - A^2 Z) - Y B^3, B^3 Z)
-__device__ NKR_PAIR_FN ProjLine proj_double(G2Proj &t, const Affine<Fq> &p)
-{
-    const Fq2 xx = sqr(t.x);
-    const Fq2 a = xx + dbl(xx);
-    const Fq2 b = dbl(t.y * t.z);
-    const Fq2 b2 = sqr(b), b3 = b2 * b;
-    const Fq2 a2z = sqr(a) * t.z;
-    const Fq2 xb2 = t.x * b2;
-    const ProjLine l{mul_fq(b * t.z, p.y), neg(mul_fq(a * t.z, p.x)), a * t.x - t.y * b};
-    const Fq2 x3 = (a2z - dbl(xb2)) * b;
-    const Fq2 y3 = a * (xb2 + dbl(xb2) - a2z) - t.y * b3;
-    t = {x3, y3, b3 * t.z};
-    return l;
-}
-
-// line through T and affine Q, T <- T + Q: with N = yQ Z - Y, D = xQ Z - X (slope N/D),
-// T + Q = ((N^2 Z - (X + xQ Z) D^2) D, N ((2X + xQ Z) D^2 - N^2 Z) - Y D^3, D^3 Z)
-__device__ NKR_PAIR_FN ProjLine proj_add(G2Proj &t, const Affine<Fq2> &q, const Affine<Fq> &p)
-{
-    const Fq2 n = q.y * t.z - t.y;
-    const Fq2 xqz = q.x * t.z;
-    const Fq2 d = xqz - t.x;
-    const Fq2 d2 = sqr(d), d3 = d2 * d;
-    const Fq2 n2z = sqr(n) * t.z;
-    const ProjLine l{mul_fq(d, p.y), neg(mul_fq(n, p.x)), n * q.x - q.y * d};
-    const Fq2 x3 = (n2z - (t.x + xqz) * d2) * d;
-    const Fq2 y3 = n * ((dbl(t.x) + xqz) * d2 - n2z) - t.y * d3;
-    t = {x3, y3, d3 * t.z};
-    return l;
-}
-
-__device__ __forceinline__ Fq6 mul_by_fq2(const Fq6 &f, const Fq2 &s) { return {f.c0 * s, f.c1 * s, f.c2 * s}; }
-
-__device__ NKR_PAIR_FN Fq12 apply_proj_line(const Fq12 &f, const ProjLine &l)
-{
-    return {mul_by_fq2(f.c0, l.c0) + mul_v(mul_by_ab(f.c1, l.a, l.b)),
-            mul_by_ab(f.c0, l.a, l.b) + mul_by_fq2(f.c1, l.c0)};
 }
 
 } // namespace nkr

@@ -1,25 +1,24 @@
 // Groth16 verification on one B200: the reference's verify
 // (protocols/groth16/common/src/protocol.cpp:96-108) for a batch of proofs of
-// one verification key, one proof per thread, and the reduced pairing as an
-// operator (libff Curve::reduced_pairing).
+// one verification key, six lanes per proof (pairing_lanes.cuh), and the reduced
+// pairing as an operator (libff Curve::reduced_pairing).
 //
 // The reference checks e(A, B) == e(alpha, beta) e(vk_x, gamma) e(C, delta)
 // with three reduced pairings, vk_x = ic[0] + sum_j x_j ic[j + 1].  Here each
-// thread runs one Miller loop over the three pairs (A, B), (-vk_x, gamma),
+// proof takes one Miller loop over the three pairs (A, B), (-vk_x, gamma),
 // (-C, delta) and one final exponentiation, and compares with the key's
 // e(alpha, beta): the same equation in GT, since the final exponentiation is a
 // homomorphism.  gamma and delta are fixed per key, so their Miller-loop lines
 // are computed once when the key is prepared; per proof only B's lines are
 // computed (homogeneous coordinates, no inversion).  vk_x is a multi-scalar
 // multiplication over the key's fixed ic points: the key holds the signed 5-bit
-// window multiples d 2^(5w) ic[j + 1] (w < 51, d = 1..16, affine), and one warp per proof
-// sums the looked-up points of its public inputs (k_vk_x, in the FP64 field)
-// before the pairing kernel runs.
+// window multiples d 2^(5w) ic[j + 1] (w < 51, d = 1..16, affine), and 8 or 32 lanes per
+// proof sum the looked-up points of its public inputs (k_vk_x) before the pairing kernel
+// runs.
 #define NKR_FIELD_MUL_OUTLINE 1
 #include <cstring>
 
-#include "field52.cuh"
-#include "pairing.cuh"
+#include "pairing_lanes.cuh"
 #include "prover.cuh"
 
 struct nkr_b200_vk {
@@ -29,7 +28,7 @@ struct nkr_b200_vk {
     nkr::DevBuf ic;    // ic[] as G1 affine (R domain)
     nkr::DevBuf lines; // kAteLines lines of gamma, then of delta
     nkr::DevBuf flags; // int[2]: gamma, delta at infinity
-    nkr::DevBuf tab;   // [n_ic - 1][51][16] affine d 2^(5w) ic[j + 1], R' = 2^260 domain
+    nkr::DevBuf tab;   // [n_ic - 1][51][16] affine d 2^(5w) ic[j + 1]
     nkr::DevBuf io;    // batch staging (grown on demand)
 };
 
@@ -39,18 +38,20 @@ namespace {
 
 constexpr size_t kProofBytes = 96 + 192 + 96; // A, B, C in libff layout
 constexpr int kIcWin = 51, kIcDig = 16;       // signed 5-bit windows of a public input
+// up to this many public inputs a proof's vk_x takes 8 lanes, beyond it a warp: 8 lanes
+// need a third of the additions for the final sum, 32 are done sooner
+constexpr uint64_t kFewInputs = 64;
 
 // libff Jacobian (X, Y, Z) -> affine; Z = 0 is infinity
 template <class F>
 __device__ __forceinline__ Affine<F> libff_to_affine(const F *p)
 {
     if (p[2].is_zero()) return Affine<F>::inf();
+    if (p[2] == F::one()) return {p[0], p[1]};
     const F zi = inverse(p[2]);
     const F zi2 = sqr(zi);
     return {p[0] * zi2, p[1] * (zi2 * zi)};
 }
-
-__device__ __forceinline__ Affine<Fq> g1_neg(const Affine<Fq> &p) { return affine_neg(p); }
 
 // gamma (lane 0) and delta (lane 1): Miller-loop lines; lanes also normalise ic
 __global__ void __launch_bounds__(32) k_vk_setup(const Fq2 *gd_jac, const Fq *ic_jac, uint64_t n_ic,
@@ -79,14 +80,7 @@ __global__ void __launch_bounds__(64) k_ic_pow(const G1Affine *ic, uint64_t n_pu
     }
 }
 
-// R = 2^256 affine -> the FP64 field's R' = 2^260 domain (stored in the Fq layout)
-__device__ __forceinline__ G1Affine affine_to_r260_storage(const G1Affine &a)
-{
-    if (a.is_inf()) return {Fq::zero(), from52(Fq52::one())};
-    return {from52(r256_to_r260(to52(a.x))), from52(r256_to_r260(to52(a.y)))};
-}
-
-// tab[(j * 51 + w) * 16 + d - 1] = d Q_{j,w} (d = 1..16), affine in the R' domain
+// tab[(j * 51 + w) * 16 + d - 1] = d Q_{j,w} (d = 1..16), affine
 __global__ void __launch_bounds__(64) k_ic_entries(const G1Xyzz *pow, uint64_t count, G1Affine *tab)
 {
     const uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -98,127 +92,141 @@ __global__ void __launch_bounds__(64) k_ic_entries(const G1Xyzz *pow, uint64_t c
         acc = xyzz_dbl(acc);
         if ((d >> b) & 1) acc = xyzz_add(acc, q);
     }
-    tab[i] = affine_to_r260_storage(xyzz_to_affine(acc));
+    tab[i] = xyzz_to_affine(acc);
 }
 
-// vk_x of proof i = ic[0] + sum_j x_ij ic[j + 1], one warp per proof: lane l sums
-// the table points of public inputs l, l + 32, ...; the warp adds its lanes'
-// sums; lane 0 writes the affine result.
-__device__ __forceinline__ Fq52 shfl_down52(const Fq52 &a, int off)
+__device__ __forceinline__ FqL shfl_down_fq(const FqL &a, int off)
 {
-    Fq52 r;
+    FqL r;
 #pragma unroll
-    for (int k = 0; k < 5; ++k) r.l[k] = __shfl_down_sync(0xffffffffu, a.l[k], off);
+    for (int k = 0; k < 8; ++k) r.v[k] = __shfl_down_sync(0xffffffffu, a.v[k], off);
     return r;
 }
-__device__ __forceinline__ Xyzz<Fq52> shfl_down_g1(const Xyzz<Fq52> &p, int off)
-{
-    return {shfl_down52(p.x, off), shfl_down52(p.y, off), shfl_down52(p.zz, off), shfl_down52(p.zzz, off)};
-}
 
-// Signed 5-bit windows, 3 blocks per SM (a 168-register budget): 22.9 K proofs/s
-// with 3,072 public inputs, against 19.4 K for unsigned 4-bit windows at the same
-// budget and 18.0 K for those at the compiler's own 214 registers and 2 blocks
-__global__ void __launch_bounds__(128, 3) k_vk_x(const G1Affine *ic, const G1Affine *tab, uint64_t n_pub,
-                                              const Fr *publics, uint64_t count, G1Affine *vk_x)
+// vk_x of proof i = ic[0] + sum_j x_ij ic[j + 1] in XYZZ coordinates, L lanes per proof: lane
+// l sums the table points of digits l, l + L, ... of all public inputs, 51 signed 5-bit
+// digits each, and the lanes' sums are added up; no inversion, the pairing takes the
+// point as it is.  With one input per lane four inputs left 28 lanes of a warp idle and
+// cost 51 dependent additions; 8 lanes per proof for few inputs keep the final sum short.
+// Digits: d_w + 15 are the 5-bit digits of x + sum_w 15 32^w, so they need no carry from
+// the windows below (the sum is below 2^255).
+template <int L>
+__global__ void __launch_bounds__(128) k_vk_x(const G1Affine *ic, const G1Affine *tab, uint64_t n_pub,
+                                              const Fr *publics, uint64_t count, G1Xyzz *vk_x)
 {
-    const uint64_t i = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (i >= count) return; // whole warps: count is per warp
-    // the FP64 field (52-bit limbs, paired products): the table holds R' values
-    Xyzz<Fq52> acc = Xyzz<Fq52>::inf();
-    for (uint64_t j = lane; j < n_pub; j += 32) {
-        const Fr x = from_mont(publics[i * n_pub + j]);
-        const G1Affine *t = tab + j * (kIcWin * kIcDig);
-        // signed digits: v = bits + carry, v > 16 -> v - 32 (x < 2^254 leaves no carry)
-        uint32_t carry = 0;
-        for (int w = 0; w < kIcWin; ++w) {
-            const int off = 5 * w, limb = off >> 5, sh = off & 31;
-            uint64_t word = x.v[limb];
-            if (limb + 1 < 8) word |= uint64_t(x.v[limb + 1]) << 32;
-            const uint32_t v = (uint32_t(word >> sh) & 31u) + carry;
-            carry = v > 16 ? 1u : 0u;
-            const int d = v > 16 ? int(v) - 32 : int(v);
-            if (d) {
-                const G1Affine e = t[w * kIcDig + (d < 0 ? -d : d) - 1];
-                const Affine<Fq52> p{to52(e.x), to52(e.y)};
-                acc = xyzz_add_affine(acc, d < 0 ? affine_neg(p) : p);
+    const uint64_t at = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) / L;
+    const uint64_t i = at < count ? at : count - 1;
+    const int lane = threadIdx.x % L;
+    Xyzz<FqL> acc = Xyzz<FqL>::inf();
+    uint64_t have = ~uint64_t(0); // public input whose biased scalar is in x
+    Fr x = Fr::zero();
+    for (uint64_t it = lane; it < n_pub * kIcWin; it += L) {
+        const uint64_t j = it / kIcWin;
+        const int w = int(it % kIcWin);
+        if (j != have) {
+            have = j;
+            x = from_mont(publics[i * n_pub + j]);
+            // sum_w 15 32^w over 51 windows: bits 5w .. 5w + 3
+            uint64_t c = 0;
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                uint32_t bias = 0;
+#pragma unroll
+                for (int b = 0; b < 32; ++b)
+                    if (32 * k + b < 5 * kIcWin && (32 * k + b) % 5 != 4) bias |= 1u << b;
+                c += uint64_t(x.v[k]) + bias;
+                x.v[k] = uint32_t(c);
+                c >>= 32;
             }
         }
+        const int off = 5 * w, limb = off >> 5, sh = off & 31;
+        uint32_t lo = 0, hi = 0;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            lo = k == limb ? x.v[k] : lo;
+            hi = k == limb + 1 ? x.v[k] : hi;
+        }
+        const int d = int(__funnelshift_r(lo, hi, sh) & 31u) - 15;
+        if (d) {
+            const G1Affine e = tab[(j * kIcWin + w) * kIcDig + (d < 0 ? -d : d) - 1];
+            const Affine<FqL> p{FqL(e.x), FqL(e.y)};
+            acc = xyzz_add_affine(acc, d < 0 ? affine_neg(p) : p);
+        }
     }
-    for (int off = 16; off; off >>= 1) acc = xyzz_add(acc, shfl_down_g1(acc, off));
-    if (lane == 0) {
-        const G1Affine i0 = affine_to_r260_storage(ic[0]);
-        const Affine<Fq52> a = xyzz_to_affine(xyzz_add_affine(acc, Affine<Fq52>{to52(i0.x), to52(i0.y)}));
-        vk_x[i] = a.is_inf() ? G1Affine::inf()
-                             : G1Affine{from52(r260_to_r256(a.x)), from52(r260_to_r256(a.y))};
+    for (int off = L / 2; off; off >>= 1)
+        acc = xyzz_add(acc, Xyzz<FqL>{shfl_down_fq(acc.x, off), shfl_down_fq(acc.y, off), shfl_down_fq(acc.zz, off),
+                                      shfl_down_fq(acc.zzz, off)});
+    if (lane == 0 && at < count) {
+        acc = xyzz_add_affine(acc, Affine<FqL>{FqL(ic[0].x), FqL(ic[0].y)});
+        vk_x[i] = acc.is_inf() ? G1Xyzz::inf()
+                               : G1Xyzz{acc.x.canon(), acc.y.canon(), acc.zz.canon(), acc.zzz.canon()};
     }
 }
 
-// reduced pairings of count (P, Q) pairs, one per thread
-__global__ void __launch_bounds__(64) k_pairing(const Fq *p_jac, const Fq2 *q_jac, uint64_t count,
-                                                Fq12 *out)
+// reduced pairings of count (P, Q) pairs, six lanes each
+__global__ void __launch_bounds__(32) k_pairing(const Fq *p_jac, const Fq2 *q_jac, uint64_t count, Fq2 *out)
 {
-    const uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= count) return;
+    __shared__ uint4 sm[kPairSmemChunks];
+    const PairGroup g(sm, threadIdx.x);
+    const uint64_t at = uint64_t(blockIdx.x) * kPairGroups + threadIdx.x / kPairLanes;
+    const uint64_t i = at < count ? at : count - 1;
     const Affine<Fq> p = libff_to_affine(p_jac + 3 * i);
     const Affine<Fq2> q = libff_to_affine(q_jac + 3 * i);
-    if (p.is_inf() || q.is_inf()) {
-        out[i] = fq12_one();
-        return;
+    if (g.m == 0) {
+        g.st(kSlQx, q.x);
+        g.st(kSlQy, q.y);
+        g.st(kSlNegPx, {neg(p.x), Fq::zero()});
+        g.st(kSlPy, {p.y, Fq::zero()});
+        g.st(kSlNegPx1, Fq2::zero());
+        g.st(kSlNegPx2, Fq2::zero());
     }
-    Fq12 f = fq12_one();
-    G2Proj t{q.x, q.y, Fq2::one()};
-    for (int b = kAteTopBit - 1; b >= 0; --b) {
-        f = sqr(f);
-        f = apply_proj_line(f, proj_double(t, p));
-        if (ate_bit(b)) f = apply_proj_line(f, proj_add(t, q, p));
-    }
-    f = apply_proj_line(f, proj_add(t, twist_frobenius(q), p));
-    f = apply_proj_line(f, proj_add(t, twist_neg_frobenius2(q), p));
-    out[i] = final_exponentiation(f);
+    __syncwarp();
+    const PairGroup::Fixed off{{nullptr, nullptr}, {false, false}};
+    // a point at infinity: all lines are 1, and so is the pairing
+    Fq2 f = g.miller(off, !p.is_inf() && !q.is_inf(), false, Fq::zero());
+    f = g.final_power(f);
+    if (g.live && at < count) out[6 * i + g.tower_index()] = f;
 }
 
-// One proof per thread: proofs[i] = A (G1), B (G2), C (G1) in libff layout;
-// vk_x[i] from k_vk_x.
-__global__ void __launch_bounds__(64) k_verify(const Fq12 *gt, const G1Affine *vk_x,
-                                               const AteLine *lines, const int *flags,
-                                               const uint8_t *proofs, uint64_t count, uint8_t *accept)
+// Six lanes per proof: proofs[i] = A (G1), B (G2), C (G1) in libff layout; vk_x[i] from
+// k_vk_x.  The line of (-vk_x, gamma) at vk_x = (X / ZZ, Y / ZZZ) is taken times ZZ ZZZ, a
+// factor in Fq that the final exponentiation removes.
+__global__ void __launch_bounds__(32) k_verify(const Fq2 *gt, const G1Xyzz *vk_x, const AteLine *lines,
+                                               const int *flags, const uint8_t *proofs, uint64_t count,
+                                               uint8_t *accept)
 {
-    const uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= count) return;
+    __shared__ uint4 sm[kPairSmemChunks];
+    const PairGroup g(sm, threadIdx.x);
+    const int group = min(int(threadIdx.x) / kPairLanes, kPairGroups - 1);
+    const uint64_t at = uint64_t(blockIdx.x) * kPairGroups + group;
+    const uint64_t i = at < count ? at : count - 1;
     const uint8_t *pr = proofs + i * kProofBytes;
     const Affine<Fq> a = libff_to_affine(reinterpret_cast<const Fq *>(pr));
     const Affine<Fq2> b = libff_to_affine(reinterpret_cast<const Fq2 *>(pr + 96));
     const Affine<Fq> c = libff_to_affine(reinterpret_cast<const Fq *>(pr + 288));
-    const Affine<Fq> nvk = g1_neg(vk_x[i]);
-    const Affine<Fq> nc = g1_neg(c);
+    const G1Xyzz vk = vk_x[i];
     const bool on1 = !a.is_inf() && !b.is_inf();
-    const bool on2 = !nvk.is_inf() && !flags[0];
-    const bool on3 = !nc.is_inf() && !flags[1];
-    const AteLine *lg = lines, *ld = lines + kAteLines;
-    Fq12 f = fq12_one();
-    G2Proj t{b.x, b.y, Fq2::one()};
-    int s = 0;
-    for (int bit = kAteTopBit - 1; bit >= 0; --bit) {
-        f = sqr(f);
-        if (on1) f = apply_proj_line(f, proj_double(t, a));
-        if (on2) f = apply_line(f, lg[s], nvk);
-        if (on3) f = apply_line(f, ld[s], nc);
-        ++s;
-        if (ate_bit(bit)) {
-            if (on1) f = apply_proj_line(f, proj_add(t, b, a));
-            if (on2) f = apply_line(f, lg[s], nvk);
-            if (on3) f = apply_line(f, ld[s], nc);
-            ++s;
-        }
+    const bool on2 = !vk.is_inf() && !flags[0];
+    const bool on3 = !c.is_inf() && !flags[1];
+    const Fq none = Fq::zero();
+    if (g.m == 0) {
+        g.st(kSlQx, b.x);
+        g.st(kSlQy, b.y);
+        g.st(kSlNegPx, {neg(a.x), none});
+        g.st(kSlPy, {a.y, none});
+    } else if (g.m == 1) {
+        g.st(kSlNegPx1, {neg(vk.x * vk.zzz), none});
+        g.st(kSlLine + 5, on2 ? Fq2{neg(vk.y * vk.zz), none} : Fq2::one());
+    } else if (g.m == 2) {
+        g.st(kSlNegPx2, {neg(c.x), none});
+        g.st(kSlLine + 10, on3 ? Fq2{neg(c.y), none} : Fq2::one());
     }
-    for (int k = 0; k < 2; ++k, ++s) {
-        if (on1) f = apply_proj_line(f, proj_add(t, k == 0 ? twist_frobenius(b) : twist_neg_frobenius2(b), a));
-        if (on2) f = apply_line(f, lg[s], nvk);
-        if (on3) f = apply_line(f, ld[s], nc);
-    }
-    accept[i] = final_exponentiation(f) == gt[0] ? 1 : 0;
+    __syncwarp();
+    const PairGroup::Fixed fx{{lines, lines + kAteLines}, {on2, on3}};
+    Fq2 f = g.miller(fx, on1, true, vk.zz * vk.zzz);
+    f = g.final_power(f);
+    const unsigned same = __ballot_sync(0xffffffffu, f == gt[g.tower_index()]);
+    if (g.live && g.m == 0 && at < count) accept[i] = ((same >> (group * kPairLanes)) & 63u) == 63u;
 }
 
 } // namespace
@@ -245,8 +253,8 @@ int nkr_b200_vk_prepare(nkr_b200_ctx *ctx, const nkr_b200_verification_key *vk, 
     NKR_CUDA(cudaMemcpyAsync(sp, vk->gamma_g2, 192, cudaMemcpyHostToDevice, st));
     NKR_CUDA(cudaMemcpyAsync(sp + 192, vk->delta_g2, 192, cudaMemcpyHostToDevice, st));
     NKR_CUDA(cudaMemcpyAsync(sp + 384, vk->ic, vk->n_ic * 96, cudaMemcpyHostToDevice, st));
-    NKR_TRY(key->gt.alloc(sizeof(Fq12), "e(alpha, beta)"));
-    NKR_CUDA(cudaMemcpyAsync(key->gt.p, vk->alpha_g1_beta_g2, sizeof(Fq12), cudaMemcpyHostToDevice, st));
+    NKR_TRY(key->gt.alloc(kFq12Bytes, "e(alpha, beta)"));
+    NKR_CUDA(cudaMemcpyAsync(key->gt.p, vk->alpha_g1_beta_g2, kFq12Bytes, cudaMemcpyHostToDevice, st));
     NKR_TRY(key->ic.alloc(vk->n_ic * sizeof(G1Affine), "ic"));
     NKR_TRY(key->lines.alloc(2 * kAteLines * sizeof(AteLine), "gamma / delta lines"));
     NKR_TRY(key->flags.alloc(2 * sizeof(int), "gamma / delta flags"));
@@ -285,21 +293,24 @@ int nkr_b200_verify_batch(nkr_b200_vk *vk, const void *public_inputs, uint64_t n
     }
     NKR_CUDA(cudaSetDevice(vk->ctx->device));
     cudaStream_t st = vk->ctx->stream;
-    // staging: proofs | public inputs | vk_x (affine) | verdicts
-    const uint64_t pb = count * kProofBytes, xb = count * n_public * 32, vb = count * sizeof(G1Affine);
+    // staging: proofs | public inputs | vk_x (XYZZ) | verdicts
+    const uint64_t pb = count * kProofBytes, xb = count * n_public * 32, vb = count * sizeof(G1Xyzz);
     NKR_TRY(vk->io.alloc(pb + xb + vb + count, "verification batch"));
     uint8_t *dp = vk->io.as<uint8_t>();
-    G1Affine *vkx = reinterpret_cast<G1Affine *>(dp + pb + xb);
+    G1Xyzz *vkx = reinterpret_cast<G1Xyzz *>(dp + pb + xb);
     uint8_t *acc = dp + pb + xb + vb;
     NKR_CUDA(cudaMemcpyAsync(dp, proofs, pb, cudaMemcpyHostToDevice, st));
     if (xb) NKR_CUDA(cudaMemcpyAsync(dp + pb, public_inputs, xb, cudaMemcpyHostToDevice, st));
-    k_vk_x<<<blocks_for(count * 32, 128), 128, 0, st>>>(vk->ic.as<G1Affine>(), vk->tab.as<G1Affine>(), n_public,
-                                                       reinterpret_cast<const Fr *>(dp + pb), count, vkx);
+    const Fr *pub = reinterpret_cast<const Fr *>(dp + pb);
+    if (n_public <= kFewInputs)
+        k_vk_x<8><<<blocks_for(count * 8, 128), 128, 0, st>>>(vk->ic.as<G1Affine>(), vk->tab.as<G1Affine>(), n_public,
+                                                              pub, count, vkx);
+    else
+        k_vk_x<32><<<blocks_for(count * 32, 128), 128, 0, st>>>(vk->ic.as<G1Affine>(), vk->tab.as<G1Affine>(),
+                                                                n_public, pub, count, vkx);
     NKR_CHECK_LAUNCH();
-    // one warp per block: at 255 registers an SM holds 8 such blocks, and a batch
-    // spreads over every SM before any SM takes a second warp
-    k_verify<<<blocks_for(count, 32), 32, 0, st>>>(vk->gt.as<Fq12>(), vkx, vk->lines.as<AteLine>(),
-                                                   vk->flags.as<int>(), dp, count, acc);
+    k_verify<<<blocks_for(count, kPairGroups), 32, 0, st>>>(vk->gt.as<Fq2>(), vkx, vk->lines.as<AteLine>(),
+                                                            vk->flags.as<int>(), dp, count, acc);
     NKR_CHECK_LAUNCH();
     NKR_CUDA(cudaMemcpyAsync(accept, acc, count, cudaMemcpyDeviceToHost, st));
     NKR_CUDA(cudaStreamSynchronize(st));
@@ -321,15 +332,15 @@ int nkr_b200_reduced_pairing(nkr_b200_ctx *ctx, const void *p_g1, const void *q_
     NKR_CUDA(cudaSetDevice(ctx->device));
     cudaStream_t st = ctx->stream;
     DevBuf buf;
-    NKR_TRY(buf.alloc(count * (96 + 192 + sizeof(Fq12)), "pairing buffers"));
+    NKR_TRY(buf.alloc(count * (96 + 192 + kFq12Bytes), "pairing buffers"));
     uint8_t *b = buf.as<uint8_t>();
     NKR_CUDA(cudaMemcpyAsync(b, p_g1, count * 96, cudaMemcpyHostToDevice, st));
     NKR_CUDA(cudaMemcpyAsync(b + count * 96, q_g2, count * 192, cudaMemcpyHostToDevice, st));
-    Fq12 *o = reinterpret_cast<Fq12 *>(b + count * 288);
-    k_pairing<<<blocks_for(count, 64), 64, 0, st>>>(reinterpret_cast<const Fq *>(b),
-                                                    reinterpret_cast<const Fq2 *>(b + count * 96), count, o);
+    Fq2 *o = reinterpret_cast<Fq2 *>(b + count * 288);
+    k_pairing<<<blocks_for(count, kPairGroups), 32, 0, st>>>(reinterpret_cast<const Fq *>(b),
+                                                             reinterpret_cast<const Fq2 *>(b + count * 96), count, o);
     NKR_CHECK_LAUNCH();
-    NKR_CUDA(cudaMemcpyAsync(out_gt, o, count * sizeof(Fq12), cudaMemcpyDeviceToHost, st));
+    NKR_CUDA(cudaMemcpyAsync(out_gt, o, count * kFq12Bytes, cudaMemcpyDeviceToHost, st));
     NKR_CUDA(cudaStreamSynchronize(st));
     return NKR_B200_OK;
 }

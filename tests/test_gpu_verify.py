@@ -143,3 +143,53 @@ def test_gpu_setup_key_verifies_its_proofs(ctx, ref):
     assert vk.verify_batch(np.stack([pub] * 4), proofs).all()
     vk.free()
     be.free()
+
+
+@pytest.mark.parametrize("count", [1, 5, 6, 11])
+def test_reduced_pairing_matches_the_oracle(ctx, orc, count):
+    """Whole, short and single groups of five pairings to a warp against the Python
+    pairing; the last pair of each call has a point at infinity."""
+    import pairing
+    rng = np.random.default_rng(51)
+    g1, g2 = orc.g1_generator(), orc.g2_generator()
+    one = O.fq_mont(1)
+    p = np.stack([np.concatenate([orc.mul_affine(1, g1, k), one]) for k in O.random_fr(count, rng)])
+    q = np.stack([np.concatenate([orc.mul_affine(2, g2, k), one, 0 * one]) for k in O.random_fr(count, rng)])
+    inf = count - 1
+    if count % 2:
+        p[inf] = np.concatenate([0 * one, one, 0 * one])
+    else:
+        q[inf] = np.concatenate([0 * one, 0 * one, one, 0 * one, 0 * one, 0 * one])
+    got = nk.reduced_pairing(ctx, p, q)
+    for i in range(min(count - 1, 3)):
+        assert np.array_equal(got[i], pairing.reduced_pairing_limbs(p[i], q[i])), i
+    assert np.array_equal(got[inf], np.concatenate([one, np.zeros(44, np.uint64)]))
+    for i in range(3, count - 1): # position in the batch does not matter
+        assert np.array_equal(got[i], nk.reduced_pairing(ctx, p[i:i + 1], q[i:i + 1])[0]), i
+
+
+@pytest.mark.parametrize("size", [2, 5])
+def test_verify_with_8_and_32_lanes_per_vk_x(ctx, size):
+    """12 and 75 public inputs lie on both sides of the vk_x lane count's limit; changed
+    inputs and unnormalised (Z != 1) proof points included."""
+    r1 = nk.generate("matmul", size, 0, seed=8)
+    pk, vkp = nk.setup(ctx, r1, O.random_fr(5, np.random.default_rng(52)))
+    be = nk.Backend(ctx)
+    be.prepare(r1, pk)
+    raw = be.prove(r1.witness)
+    rs = O.random_fr(14, np.random.default_rng(53)).reshape(7, 2, 4)
+    proofs = np.stack([_proof_array(be.blind(raw, r, s)) for r, s in rs])
+    publics = np.stack([np.ascontiguousarray(r1.witness[1:1 + r1.public_inputs])] * 7)
+    want = np.ones(7, bool)
+    for i, j in ((1, 0), (3, r1.public_inputs - 1), (6, 1)):
+        publics[i, j] = O.fr_mont(O.fr_int(publics[i, j]) + 1)
+        want[i] = False
+    # A and C of proof 2 as (X z^2, Y z^3, z)
+    z = 0x1234567
+    for at in (0, 36):
+        x, y = O.fq_int(proofs[2, at:at + 4]), O.fq_int(proofs[2, at + 4:at + 8])
+        proofs[2, at:at + 12] = np.concatenate([O.fq_mont(x * z * z), O.fq_mont(y * z**3), O.fq_mont(z)])
+    vk = nk.VerifyingKey(ctx, vkp["alpha_g1_beta_g2"], vkp["gamma_g2"], vkp["delta_g2"], vkp["ic"])
+    assert np.array_equal(vk.verify_batch(publics, proofs), want)
+    vk.free()
+    be.free()
