@@ -14,6 +14,15 @@ namespace {
 constexpr size_t kOutOffset[kNumMsm] = {0, 96, 192, 288, 384}; // A, B1, L, H, B2
 // issue order of the witness MSMs: the G2 MSM (longest) first
 constexpr int kWitnessOrder[4] = {kMsmB2, kMsmA, kMsmB1, kMsmL};
+// Repeated witness values go through the class path (msm.cuh) only for circuits of more
+// variables than this.  It is a chain of some forty dependent small launches, which takes
+// longer than the additions that it saves in a small prove.  Measured, class path on / off,
+// one prove with blinding (batch of 8 proofs): poseidon of 4, 16 and 64 hashes (2^11, 2^13
+// and 2^15 variables) 1.97 / 0.96, 2.12 / 1.15 and 2.45 / 2.26 ms (4.10 / 1.64, 6.63 / 3.02
+// and 10.1 / 7.3 ms); 256 hashes (2^17) 3.47 / 4.73 ms (20.6 / 21.4 ms); 2,048 (2^20)
+// 10.0 / 17.2 ms.  Without repeated values the path only costs: matmul 32 (2^16)
+// 2.02 / 1.58 ms, sql-aggregate 256 (2^18) 8.78 / 7.71 ms.
+constexpr uint64_t kClassColsMin = uint64_t(1) << 16;
 
 } // namespace
 
@@ -162,10 +171,12 @@ int slot_add(nkr_b200_key *key)
     }
     NKR_TRY(msm_sort_alloc(sl->sort_h, key->bases[kMsmH].shape));
     bytes += sl->sort_h.device_bytes();
-    NKR_TRY(msm_dedup_alloc(sl->dedup, key->cols));
-    bytes += sl->dedup.device_bytes();
     for (int k = 0; k < kNumMsm; ++k) {
         if (!key->classes[k]) continue;
+        if (!sl->dedup.cols) {
+            NKR_TRY(msm_dedup_alloc(sl->dedup, key->cols));
+            bytes += sl->dedup.device_bytes();
+        }
         NKR_TRY(msm_class_sort_alloc(sl->csort[k], key->bases[k].shape.n));
         bytes += sl->csort[k].device_bytes();
         NKR_TRY(msm_class_acc_alloc(sl->cacc[k], key->bases[k].group, key->bases[k].shape.n));
@@ -225,11 +236,13 @@ int prove_issue(nkr_b200_key *key, ProveSlot *sl, bool timed, bool blind_tables)
     if (timed) NKR_CUDA(cudaEventRecord(sl->ev_t[1], s0));
     // witness MSMs on their own streams, overlapping the H chain; one digit sort
     // of z (gathered through the bases' support) per distinct support
-    // classes of repeated witness values (main stream), then the digit sorts
-    // without the class members and the class members of each support
-    NKR_CUDA(cudaStreamWaitEvent(sl->cls[kMsmH], sl->ev_z, 0));
-    NKR_TRY(msm_dedup_run(sl->dedup, z, sl->cls[kMsmH]));
-    NKR_CUDA(cudaEventRecord(sl->ev_dedup, sl->cls[kMsmH]));
+    // classes of repeated witness values, then the digit sorts without the class
+    // members and the class members of each support
+    if (sl->dedup.cols) {
+        NKR_CUDA(cudaStreamWaitEvent(sl->cls[kMsmH], sl->ev_z, 0));
+        NKR_TRY(msm_dedup_run(sl->dedup, z, sl->cls[kMsmH]));
+        NKR_CUDA(cudaEventRecord(sl->ev_dedup, sl->cls[kMsmH]));
+    }
     for (int g = 0; g < key->n_sorts; ++g) {
         const int o = key->sort_stream[g];
         const bool cls = key->classes[o];
@@ -430,7 +443,7 @@ int key_prepare(nkr_b200_ctx *ctx, const nkr_b200_circuit *c, const nkr_b200_pro
     NKR_PREP(msm_bases_build(key->bases[kMsmH], 1, pk->h_query, false, c->rows, true, ch, true, st));
     // MSMs with the same support (and so the same window shape) and the same use
     // of the class path share a digit sort
-    for (int k : kWitnessOrder) key->classes[k] = true;
+    for (int k : kWitnessOrder) key->classes[k] = c->cols > kClassColsMin;
     key->n_sorts = 0;
     for (int k : kWitnessOrder) {
         int g = -1;

@@ -217,3 +217,39 @@ def test_prove_repeated_witness_values(ctx, ref, tmp_path):
     be.prove(r1.witness)
     assert bytes(be.prove(w)) == bytes(raw)
     be.free()
+
+
+@pytest.mark.parametrize("size", [32, 40])
+def test_prove_of_repeated_values_matches_plain_msms(ctx, size):
+    """matmul 32 has 2^16 variables (no class path), matmul 40 2^17 (class path): a crafted
+    witness with more classes than one prove takes, groups below the minimum, large classes,
+    negations and zeros gives the points of plain MSMs over the key's queries."""
+    r1 = nk.generate("matmul", size, 0, seed=31)
+    pk, _ = nk.setup(ctx, r1, O.random_fr(5, np.random.default_rng(78)))
+    rng = np.random.default_rng(79)
+    w = O.random_fr(r1.cols, rng)
+    w[0] = O.fr_mont(1)
+    pos = rng.permutation(np.arange(1, r1.cols))
+    vals = O.random_fr(4400, rng)
+    sizes = [4] * 4200 + [3] * 100 + [500] * 10 + [8] * 10
+    k = 0
+    for v, m in zip(vals, sizes):
+        w[pos[k:k + m]] = v
+        k += m
+    for v in vals[4310:4320]:
+        w[pos[k:k + 8]] = O.int_to_limbs((O.R - O.limbs_to_int(v)) % O.R)
+        k += 8
+    w[pos[k:k + 2000]] = 0
+    be = nk.Backend(ctx)
+    be.prepare(r1, pk)
+    raw = be.prove(w)
+    assert bytes(be.prove(w)) == bytes(raw)
+    for name, field, group in (("a_query", "ar", 1), ("b_g1_query", "bs1", 1), ("l_query", "zk", 1),
+                               ("b_g2_query", "bs2", 2)):
+        b = nk.MsmBases(ctx, group, pk[name])
+        want, _ = b.run(w)
+        b.free()
+        assert np.frombuffer(bytes(getattr(raw, field)), np.uint64).tolist() == want.tolist(), name
+    be.prove(r1.witness)
+    assert bytes(be.prove(w)) == bytes(raw)
+    be.free()
