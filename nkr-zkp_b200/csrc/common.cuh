@@ -52,6 +52,17 @@ extern std::atomic<unsigned long long> g_kernel_launches;
         }                                                                                       \
     } while (0)
 
+// Records a timing event; under stream capture it becomes an event record node, so that
+// replays of the graph time themselves.
+inline cudaError_t record_timing(cudaEvent_t ev, cudaStream_t st)
+{
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    const cudaError_t e = cudaStreamIsCapturing(st, &cs);
+    if (e != cudaSuccess) return e;
+    return cs == cudaStreamCaptureStatusActive ? cudaEventRecordWithFlags(ev, st, cudaEventRecordExternal)
+                                               : cudaEventRecord(ev, st);
+}
+
 // Device allocation with an explicit admission check against free HBM.
 int device_alloc(void **p, size_t bytes, const char *what);
 

@@ -892,10 +892,10 @@ int acc_level1_t(const MsmBases &bs, const MsmSort &s, MsmAcc &a, cudaStream_t s
     // no bucket clearing: a bucket is read only after the kernel that wrote it
     const uint64_t segs = sh.segments_max();
     const uint32_t *offsets = s.offsets.as<uint32_t>();
-    if (a.timing) NKR_CUDA(cudaEventRecord(a.ev_acc[0], st));
+    if (a.timing) NKR_CUDA(record_timing(a.ev_acc[0], st));
     NKR_TRY(launch_level1<F>(segs, offsets, s.entries.as<uint32_t>(), bs.pts.as<Affine<F>>(), sh.nb,
                              uint32_t(sh.k1), a.partials.as<Xyzz<F>>(), a.buckets.as<Xyzz<F>>(), a.fix, st));
-    if (a.timing) NKR_CUDA(cudaEventRecord(a.ev_acc[1], st));
+    if (a.timing) NKR_CUDA(record_timing(a.ev_acc[1], st));
     return NKR_B200_OK;
 }
 
@@ -957,7 +957,7 @@ int reduce_run(const MsmBases &bs, const MsmSort &s, MsmAcc &a, void *out_dev, c
         offsets, sh.nb, a.partials.as<Xyzz<F>>(), a.buckets.as<Xyzz<F>>(), items, L, uint32_t(sh.k1), bufs_a[0],
         bufs_r[0]);
     NKR_CHECK_LAUNCH();
-    if (a.timing) NKR_CUDA(cudaEventRecord(a.ev_acc[3], st));
+    if (a.timing) NKR_CUDA(record_timing(a.ev_acc[3], st));
     const Xyzz<F> *a_in = bufs_a[0];
     const Xyzz<F> *r_in = bufs_r[0];
     int flip = 1;
@@ -978,7 +978,7 @@ int reduce_run(const MsmBases &bs, const MsmSort &s, MsmAcc &a, void *out_dev, c
     k_finalize<F><<<1, sets <= 8 ? 32 : 4 * kFinalSets, 4 * kFinalSets * sizeof(QF<F>), st>>>(
         a_in, r_in, int(sets), sh.c, static_cast<F *>(out_dev));
     NKR_CHECK_LAUNCH();
-    if (a.timing) NKR_CUDA(cudaEventRecord(a.ev_acc[4], st));
+    if (a.timing) NKR_CUDA(record_timing(a.ev_acc[4], st));
     return NKR_B200_OK;
 }
 
@@ -1002,7 +1002,7 @@ int acc_tail_t(const MsmBases &bs, const MsmSort &s, MsmAcc &a, void *out_dev, c
 {
     NKR_TRY(fixup_t<F>(bs.shape, s.offsets.as<uint32_t>(), a.partials.as<Xyzz<F>>(), a.buckets.as<Xyzz<F>>(), a.fix,
                        st));
-    if (a.timing) NKR_CUDA(cudaEventRecord(a.ev_acc[2], st));
+    if (a.timing) NKR_CUDA(record_timing(a.ev_acc[2], st));
     return reduce_run<F>(bs, s, a, out_dev, st);
 }
 

@@ -73,8 +73,8 @@ ProveSlot::~ProveSlot()
 {
     for (auto s : st)
         if (s) cudaStreamSynchronize(s);
-    if (graph_exec) cudaGraphExecDestroy(graph_exec);
-    if (graph) cudaGraphDestroy(graph);
+    batch.release();
+    single.release();
     for (auto s : tail)
         if (s) cudaStreamSynchronize(s);
     for (auto s : cls)
@@ -226,14 +226,14 @@ int prove_issue(nkr_b200_key *key, ProveSlot *sl, bool timed, bool blind_tables)
     Fr *z = sl->z.as<Fr>();
     Fr *az = sl->az.as<Fr>(), *bz = sl->bz.as<Fr>(), *cz = sl->cz.as<Fr>(), *h = sl->h.as<Fr>();
     uint8_t *out = sl->out.as<uint8_t>();
-    if (timed) NKR_CUDA(cudaEventRecord(sl->ev_t[0], s0));
+    if (timed) NKR_CUDA(record_timing(sl->ev_t[0], s0));
     for (auto &a : sl->acc) a.timing = timed; // phase events of each MSM (timed proves only)
     const CsrDevice *mats[3] = {&key->mat[0], &key->mat[1], &key->mat[2]};
     Fr *ys[3] = {az, bz, cz};
     Fr *prods[3] = {sl->spmv_prod[0].as<Fr>(), sl->spmv_prod[1].as<Fr>(), sl->spmv_prod[2].as<Fr>()};
     NKR_TRY(spmv_multi(mats, 3, z, ys, prods, s0));
     NKR_CUDA(cudaEventRecord(sl->ev_z, s0));
-    if (timed) NKR_CUDA(cudaEventRecord(sl->ev_t[1], s0));
+    if (timed) NKR_CUDA(record_timing(sl->ev_t[1], s0));
     // witness MSMs on their own streams, overlapping the H chain; one digit sort
     // of z (gathered through the bases' support) per distinct support
     // classes of repeated witness values, then the digit sorts without the class
@@ -270,7 +270,7 @@ int prove_issue(nkr_b200_key *key, ProveSlot *sl, bool timed, bool blind_tables)
             NKR_CUDA(cudaStreamWaitEvent(sl->tail[k], sl->ev_cls[k], 0));
             NKR_TRY(msm_result_add(key->bases[k].group, out + kOutOffset[k], sl->cacc[k].out.p, sl->tail[k]));
         }
-        if (timed) NKR_CUDA(cudaEventRecord(sl->ev_msm_end[k], sl->tail[k]));
+        if (timed) NKR_CUDA(record_timing(sl->ev_msm_end[k], sl->tail[k]));
         NKR_CUDA(cudaEventRecord(sl->ev_done[k], sl->tail[k]));
         return NKR_B200_OK;
     };
@@ -286,7 +286,7 @@ int prove_issue(nkr_b200_key *key, ProveSlot *sl, bool timed, bool blind_tables)
         }
         NKR_TRY(fr_quotient_pointwise(az, bz, cz, h, rows, cst + kConstZinv, sc));
         NKR_TRY(ntt_dif(T, h, true, nullptr, T.t2.as<Fr>(), nullptr, sc));
-        if (timed) NKR_CUDA(cudaEventRecord(sl->ev_t[2], sc));
+        if (timed) NKR_CUDA(record_timing(sl->ev_t[2], sc));
         NKR_TRY(msm_sort_run(key->bases[kMsmH].shape, sl->sort_h, h, sc));
         NKR_CUDA(cudaEventRecord(sl->ev_hsorted, sc));
         return NKR_B200_OK;
@@ -306,55 +306,62 @@ int prove_issue(nkr_b200_key *key, ProveSlot *sl, bool timed, bool blind_tables)
         NKR_CUDA(cudaEventRecord(sl->ev_done[kMsmA], sl->tail[kMsmA]));
     }
     NKR_CUDA(cudaStreamWaitEvent(s0, sl->ev_done[kMsmH], 0));
-    if (timed) NKR_CUDA(cudaEventRecord(sl->ev_t[3], s0));
+    if (timed) NKR_CUDA(record_timing(sl->ev_t[3], s0));
     for (int k : kWitnessOrder) NKR_CUDA(cudaStreamWaitEvent(s0, sl->ev_done[k], 0));
-    if (timed) NKR_CUDA(cudaEventRecord(sl->ev_t[4], s0));
+    if (timed) NKR_CUDA(record_timing(sl->ev_t[4], s0));
     return NKR_B200_OK;
 }
 
-int slot_capture(nkr_b200_key *key, ProveSlot *sl)
+namespace {
+
+// Captures prove_issue on a slot's streams into a graph.  by_node: its kernels run at the
+// priorities of the streams they were issued on, else at the launch stream's.
+int capture_prove(nkr_b200_key *key, ProveSlot *sl, bool timed, bool blind_tables, bool by_node, ProveGraph *out)
 {
-    if (sl->graph_exec) return NKR_B200_OK;
     NKR_CUDA(cudaSetDevice(key->ctx->device));
     for (auto s : sl->st) NKR_CUDA(cudaStreamSynchronize(s));
     for (auto s : sl->tail) NKR_CUDA(cudaStreamSynchronize(s));
     for (auto s : sl->cls) NKR_CUDA(cudaStreamSynchronize(s));
     NKR_CUDA(cudaStreamSynchronize(sl->chain));
     cudaStream_t s0 = sl->main();
-    const unsigned long long before = g_kernel_launches.load();
     NKR_CUDA(cudaStreamBeginCapture(s0, cudaStreamCaptureModeRelaxed));
-    const int s = prove_issue(key, sl, false, false);
+    const int s = prove_issue(key, sl, timed, blind_tables);
     cudaGraph_t g = nullptr;
     const cudaError_t e = cudaStreamEndCapture(s0, &g);
-    // capturing records kernels, it launches none
-    g_kernel_launches.fetch_sub(g_kernel_launches.load() - before);
     if (s != NKR_B200_OK || e != cudaSuccess) {
         if (g) cudaGraphDestroy(g);
         cudaGetLastError();
         if (s == NKR_B200_OK) set_error("prove graph capture failed: %s", cudaGetErrorString(e));
         return s != NKR_B200_OK ? s : NKR_B200_ECUDA;
     }
+    out->graph = g;
     size_t nn = 0;
     NKR_CUDA(cudaGraphGetNodes(g, nullptr, &nn));
     std::vector<cudaGraphNode_t> nodes(nn);
     NKR_CUDA(cudaGraphGetNodes(g, nodes.data(), &nn));
-    unsigned long long kernels = 0;
+    out->kernels = 0;
     for (auto nd : nodes) {
         cudaGraphNodeType t;
         NKR_CUDA(cudaGraphNodeGetType(nd, &t));
-        kernels += t == cudaGraphNodeTypeKernel;
+        out->kernels += t == cudaGraphNodeTypeKernel;
     }
-    cudaGraphExec_t ex = nullptr;
-    const cudaError_t ei = cudaGraphInstantiate(&ex, g, 0);
+    g_kernel_launches.fetch_sub(out->kernels); // recorded and counted, not launched
+    const cudaError_t ei = cudaGraphInstantiate(&out->exec, g, by_node ? cudaGraphInstantiateFlagUseNodePriority : 0);
     if (ei != cudaSuccess) {
-        cudaGraphDestroy(g);
+        out->exec = nullptr;
         set_error("prove graph instantiation failed: %s", cudaGetErrorString(ei));
         return NKR_B200_ECUDA;
     }
-    sl->graph = g;
-    sl->graph_exec = ex;
-    sl->graph_kernels = kernels;
     return NKR_B200_OK;
+}
+
+} // namespace
+
+int slot_capture(nkr_b200_key *key, ProveSlot *sl)
+{
+    if (sl->batch.exec) return NKR_B200_OK;
+    sl->batch.release();
+    return capture_prove(key, sl, false, false, false, &sl->batch);
 }
 
 int slot_upload_witness(nkr_b200_key *key, ProveSlot *sl, const void *witness)
@@ -383,8 +390,8 @@ int slot_upload_witness(nkr_b200_key *key, ProveSlot *sl, const void *witness)
 
 int slot_launch(ProveSlot *sl, cudaStream_t launch)
 {
-    NKR_CUDA(cudaGraphLaunch(sl->graph_exec, launch ? launch : sl->main()));
-    g_kernel_launches.fetch_add(sl->graph_kernels, std::memory_order_relaxed);
+    NKR_CUDA(cudaGraphLaunch(sl->batch.exec, launch ? launch : sl->main()));
+    g_kernel_launches.fetch_add(sl->batch.kernels, std::memory_order_relaxed);
     return NKR_B200_OK;
 }
 
@@ -500,7 +507,22 @@ int key_prove(nkr_b200_key *key, const void *witness, uint64_t n, nkr_b200_raw_p
     cudaStream_t s0 = sl->main();
     // s0 is ordered after the previous prove's joins, so z is free to overwrite
     NKR_CUDA(cudaMemcpyAsync(sl->z.p, witness, n * 32, copy_kind_from(witness), s0));
-    NKR_TRY(prove_issue(key, sl, true, true));
+    // The first prove of a key issues its launches, the second captures them as well: a
+    // prove is some 150 launches on 17 streams, about 0.7 ms of host work, and a program
+    // that proves once does not pay for the capture.  Replayed, a prove and blinding of a
+    // 16-step circuit takes 0.71 ms (issued 0.77), of matmul 32 1.49 ms (1.53), of 2^20
+    // constraints 10.03 ms (10.17).
+    if (sl->proves == 0) {
+        NKR_TRY(prove_issue(key, sl, true, true));
+    } else {
+        if (!sl->single.exec) {
+            sl->single.release();
+            NKR_TRY(capture_prove(key, sl, true, true, true, &sl->single));
+        }
+        NKR_CUDA(cudaGraphLaunch(sl->single.exec, s0));
+        g_kernel_launches.fetch_add(sl->single.kernels, std::memory_order_relaxed);
+    }
+    ++sl->proves;
     NKR_CUDA(cudaMemcpyAsync(sl->pinned_out, sl->out.p, kOutBytes, cudaMemcpyDeviceToHost, s0));
     NKR_CUDA(cudaStreamSynchronize(s0));
     normalize_raw(sl->pinned_out);

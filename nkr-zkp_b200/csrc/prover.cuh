@@ -52,6 +52,20 @@ enum { kMsmA = 0, kMsmB1 = 1, kMsmL = 2, kMsmH = 3, kMsmB2 = 4, kNumMsm = 5 };
 constexpr size_t kOutBytes = 4 * 96 + 192; // ar, bs1, zk, qz (G1) + bs2 (G2), libff layout
 constexpr size_t kBlindStage = 1280;       // pinned staging of one blinding, after the results
 
+// A captured prove (witness already in the slot's z) and the kernels of one replay
+struct ProveGraph {
+    cudaGraph_t graph = nullptr;
+    cudaGraphExec_t exec = nullptr;
+    unsigned long long kernels = 0;
+    void release()
+    {
+        if (exec) cudaGraphExecDestroy(exec);
+        if (graph) cudaGraphDestroy(graph);
+        exec = nullptr;
+        graph = nullptr;
+    }
+};
+
 struct ProveSlot {
     MsmSort sort_w[4]; // witness digit sorts, one per distinct support
     MsmSort sort_h;    // digit sort of H
@@ -76,10 +90,11 @@ struct ProveSlot {
     cudaEvent_t ev_z = nullptr, ev_sorted[4] = {}, ev_done[kNumMsm] = {};
     cudaEvent_t ev_t[5] = {};
     cudaEvent_t ev_msm_end[kNumMsm] = {}; // timed proves: each MSM's end on its stream
-    // the prove as a graph (witness already in z); kernels launched per replay
-    cudaGraph_t graph = nullptr;
-    cudaGraphExec_t graph_exec = nullptr;
-    unsigned long long graph_kernels = 0;
+    // the prove as a graph: of batches and the server, whose kernels run at the priority of
+    // the stream it is launched into; and of nkr_b200_prove (slot 0: stage events, blinding
+    // tables), whose kernels keep their streams' priorities
+    ProveGraph batch, single;
+    uint64_t proves = 0; // nkr_b200_prove calls on this slot
     // pinned staging: witness double buffer (pageable inputs) and results
     void *pinned_wit[2] = {nullptr, nullptr};
     cudaEvent_t ev_wit[2] = {nullptr, nullptr};
