@@ -242,20 +242,16 @@ int nkr_b200_ntt(nkr_b200_ctx *ctx, int op, void *data, uint64_t n)
     Fr *res = pb;
     switch (op) {
     case 0: // FFT
-        NKR_TRY(ntt_dif(*T, pa, false, nullptr, nullptr, nullptr, st));
-        NKR_TRY(ntt_bitrev_permute(pa, pb, n, nullptr, nullptr, st));
+        NKR_TRY(ntt_dif_natural(*T, pa, pb, false, nullptr, nullptr, nullptr, st));
         break;
     case 1: // iFFT
-        NKR_TRY(ntt_dif(*T, pa, true, nullptr, nullptr, nullptr, st));
-        NKR_TRY(ntt_bitrev_permute(pa, pb, n, nullptr, c + kConstNinv, st));
+        NKR_TRY(ntt_dif_natural(*T, pa, pb, true, nullptr, nullptr, c + kConstNinv, st));
         break;
     case 2: // cosetFFT
-        NKR_TRY(ntt_dif(*T, pa, false, T->gpow.as<Fr>(), nullptr, nullptr, st));
-        NKR_TRY(ntt_bitrev_permute(pa, pb, n, nullptr, nullptr, st));
+        NKR_TRY(ntt_dif_natural(*T, pa, pb, false, T->gpow.as<Fr>(), nullptr, nullptr, st));
         break;
     case 3: // icosetFFT
-        NKR_TRY(ntt_dif(*T, pa, true, nullptr, nullptr, nullptr, st));
-        NKR_TRY(ntt_bitrev_permute(pa, pb, n, T->t2.as<Fr>(), nullptr, st));
+        NKR_TRY(ntt_dif_natural(*T, pa, pb, true, nullptr, T->t2.as<Fr>(), nullptr, st));
         break;
     case 4: // divide_by_Z_on_coset
         NKR_TRY(fr_scale_const(pa, n, c + kConstZinv, st));
@@ -301,20 +297,16 @@ int nkr_b200_ntt_device(nkr_b200_ctx *ctx, int op, void *in, void *out, uint64_t
     Fr *pa = static_cast<Fr *>(in), *pb = static_cast<Fr *>(out);
     switch (op) {
     case 0:
-        NKR_TRY(ntt_dif(*T, pa, false, nullptr, nullptr, nullptr, st));
-        NKR_TRY(ntt_bitrev_permute(pa, pb, n, nullptr, nullptr, st));
+        NKR_TRY(ntt_dif_natural(*T, pa, pb, false, nullptr, nullptr, nullptr, st));
         break;
     case 1:
-        NKR_TRY(ntt_dif(*T, pa, true, nullptr, nullptr, nullptr, st));
-        NKR_TRY(ntt_bitrev_permute(pa, pb, n, nullptr, c + kConstNinv, st));
+        NKR_TRY(ntt_dif_natural(*T, pa, pb, true, nullptr, nullptr, c + kConstNinv, st));
         break;
     case 2:
-        NKR_TRY(ntt_dif(*T, pa, false, T->gpow.as<Fr>(), nullptr, nullptr, st));
-        NKR_TRY(ntt_bitrev_permute(pa, pb, n, nullptr, nullptr, st));
+        NKR_TRY(ntt_dif_natural(*T, pa, pb, false, T->gpow.as<Fr>(), nullptr, nullptr, st));
         break;
     case 3:
-        NKR_TRY(ntt_dif(*T, pa, true, nullptr, nullptr, nullptr, st));
-        NKR_TRY(ntt_bitrev_permute(pa, pb, n, T->t2.as<Fr>(), nullptr, st));
+        NKR_TRY(ntt_dif_natural(*T, pa, pb, true, nullptr, T->t2.as<Fr>(), nullptr, st));
         break;
     case 4:
         NKR_TRY(fr_scale_const(pa, n, c + kConstZinv, st));

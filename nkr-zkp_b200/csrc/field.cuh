@@ -163,8 +163,8 @@ __device__ __forceinline__ Fp<P> operator-(const Fp<P> &a, const Fp<P> &b)
         "addc.cc.u32 %5, %5, %13;\n\t"
         "addc.cc.u32 %6, %6, %14;\n\t"
         "addc.u32    %7, %7, %15;"
-        : "+r"(r.v[0]), "+r"(r.v[1]), "+r"(r.v[2]), "+r"(r.v[3]), "+r"(r.v[4]), "+r"(r.v[5]),
-          "+r"(r.v[6]), "+r"(r.v[7])
+        : "+&r"(r.v[0]), "+&r"(r.v[1]), "+&r"(r.v[2]), "+&r"(r.v[3]), "+&r"(r.v[4]), "+&r"(r.v[5]),
+          "+&r"(r.v[6]), "+&r"(r.v[7])
         : "r"(P::P0 & br), "r"(P::P1 & br), "r"(P::P2 & br), "r"(P::P3 & br), "r"(P::P4 & br),
           "r"(P::P5 & br), "r"(P::P6 & br), "r"(P::P7 & br));
     return r;
@@ -201,8 +201,8 @@ __device__ __forceinline__ Fp<P> dbl(const Fp<P> &a)
         "madc.hi.cc.u32 %6, %14, %17, %6;\n\t"                                                 \
         "madc.hi.cc.u32 %7, %15, %17, %7;\n\t"                                                 \
         "madc.hi.u32    %8, %16, %17, %8;"                                                     \
-        : "+r"(t0), "+r"(t1), "+r"(t2), "+r"(t3), "+r"(t4), "+r"(t5), "+r"(t6), "+r"(t7),      \
-          "+r"(t8)                                                                             \
+        : "+&r"(t0), "+&r"(t1), "+&r"(t2), "+&r"(t3), "+&r"(t4), "+&r"(t5), "+&r"(t6), "+&r"(t7),      \
+          "+&r"(t8)                                                                             \
         : "r"(a.v[0]), "r"(a.v[1]), "r"(a.v[2]), "r"(a.v[3]), "r"(a.v[4]), "r"(a.v[5]),        \
           "r"(a.v[6]), "r"(a.v[7]), "r"(bi));                                                  \
     {                                                                                          \
@@ -224,8 +224,8 @@ __device__ __forceinline__ Fp<P> dbl(const Fp<P> &a)
             "madc.hi.cc.u32 %6, %9, %15, %6;\n\t"                                              \
             "madc.hi.cc.u32 %7, %9, %16, %7;\n\t"                                              \
             "madc.hi.u32    %8, %9, %17, %8;"                                                  \
-            : "+r"(t0), "+r"(t1), "+r"(t2), "+r"(t3), "+r"(t4), "+r"(t5), "+r"(t6), "+r"(t7),  \
-              "+r"(t8)                                                                         \
+            : "+&r"(t0), "+&r"(t1), "+&r"(t2), "+&r"(t3), "+&r"(t4), "+&r"(t5), "+&r"(t6), "+&r"(t7),  \
+              "+&r"(t8)                                                                         \
             : "r"(m), "n"(P::P0), "n"(P::P1), "n"(P::P2), "n"(P::P3), "n"(P::P4), "n"(P::P5),  \
               "n"(P::P6), "n"(P::P7));                                                         \
     }                                                                                          \
@@ -302,8 +302,8 @@ __device__ __forceinline__ void eo_mad(uint32_t *x, uint32_t &c, uint32_t a0, ui
         "madc.lo.cc.u32 %6, %12, %13, %6;\n\t"
         "madc.hi.cc.u32 %7, %12, %13, %7;\n\t"
         "addc.u32       %8, %8, 0;"
-        : "+r"(x[0]), "+r"(x[1]), "+r"(x[2]), "+r"(x[3]), "+r"(x[4]), "+r"(x[5]), "+r"(x[6]),
-          "+r"(x[7]), "+r"(c)
+        : "+&r"(x[0]), "+&r"(x[1]), "+&r"(x[2]), "+&r"(x[3]), "+&r"(x[4]), "+&r"(x[5]), "+&r"(x[6]),
+          "+&r"(x[7]), "+&r"(c)
         : "r"(a0), "r"(a2), "r"(a4), "r"(a6), "r"(b));
 }
 
@@ -319,7 +319,7 @@ __device__ __forceinline__ void eo_mad_fit(uint32_t *x, uint32_t a0, uint32_t a2
         "madc.hi.cc.u32 %5, %10, %12, %5;\n\t"
         "madc.lo.cc.u32 %6, %11, %12, %6;\n\t"
         "madc.hi.u32    %7, %11, %12, %7;"
-        : "+r"(x[0]), "+r"(x[1]), "+r"(x[2]), "+r"(x[3]), "+r"(x[4]), "+r"(x[5]), "+r"(x[6]), "+r"(x[7])
+        : "+&r"(x[0]), "+&r"(x[1]), "+&r"(x[2]), "+&r"(x[3]), "+&r"(x[4]), "+&r"(x[5]), "+&r"(x[6]), "+&r"(x[7])
         : "r"(a0), "r"(a2), "r"(a4), "r"(a6), "r"(b));
 }
 
@@ -341,8 +341,8 @@ __device__ __forceinline__ void eo_mad_word(uint32_t *x, uint32_t &c, uint32_t w
         "madc.hi.cc.u32 %7, %12, %13, %7;\n\t"
         "addc.u32       %8, 0, 0;\n\t"
         "}"
-        : "+r"(x[0]), "+r"(x[1]), "+r"(x[2]), "+r"(x[3]), "+r"(x[4]), "+r"(x[5]), "+r"(x[6]),
-          "+r"(x[7]), "=r"(c)
+        : "+&r"(x[0]), "+&r"(x[1]), "+&r"(x[2]), "+&r"(x[3]), "+&r"(x[4]), "+&r"(x[5]), "+&r"(x[6]),
+          "+&r"(x[7]), "=r"(c)
         : "r"(a0), "r"(a2), "r"(a4), "r"(a6), "r"(b), "r"(w));
 }
 
@@ -376,7 +376,7 @@ __device__ __forceinline__ void add_words_carry(uint32_t *r, const uint32_t *x, 
         "addc.cc.u32 %7, %16, %24;\n\t"
         "addc.u32    %8, 0, 0;"
         : "=&r"(r[0]), "=&r"(r[1]), "=&r"(r[2]), "=&r"(r[3]), "=&r"(r[4]), "=&r"(r[5]), "=&r"(r[6]),
-          "=&r"(r[7]), "+r"(c)
+          "=&r"(r[7]), "+&r"(c)
         : "r"(x[0]), "r"(x[1]), "r"(x[2]), "r"(x[3]), "r"(x[4]), "r"(x[5]), "r"(x[6]), "r"(x[7]),
           "r"(y[0]), "r"(y[1]), "r"(y[2]), "r"(y[3]), "r"(y[4]), "r"(y[5]), "r"(y[6]), "r"(y[7]));
 }
@@ -408,7 +408,7 @@ __device__ __forceinline__ void sub_words16(uint32_t *r, const uint32_t *x, cons
         "subc.cc.u32 %6, %15, %23;\n\t"
         "subc.u32    %7, %16, %24;"
         : "=&r"(r[8]), "=&r"(r[9]), "=&r"(r[10]), "=&r"(r[11]), "=&r"(r[12]), "=&r"(r[13]), "=&r"(r[14]),
-          "=&r"(r[15]), "+r"(br)
+          "=&r"(r[15]), "+&r"(br)
         : "r"(x[8]), "r"(x[9]), "r"(x[10]), "r"(x[11]), "r"(x[12]), "r"(x[13]), "r"(x[14]), "r"(x[15]),
           "r"(y[8]), "r"(y[9]), "r"(y[10]), "r"(y[11]), "r"(y[12]), "r"(y[13]), "r"(y[14]), "r"(y[15]));
 }
@@ -545,76 +545,99 @@ __device__ Fp<P> inverse(const Fp<P> &a)
 }
 
 // ---------------------------------------------------------------------------
-// FqL: Fq values in [0, 2p), the compute type of the G1 MSM.  A product of two such
-// values is below 1.76 p as it stands (mont_mul), so products skip the conditional
-// subtraction; additions and subtractions work modulo 2p.  Zero tests accept 0 and p.
-// Values are made canonical when they leave for memory (canon()).
+// FpL: values in [0, 2p), the compute type of the G1 MSM (FqL) and of the transforms
+// (FrL).  A product of two such values is below 1.76 p as it stands (mont_mul), so
+// products skip the conditional subtraction; additions and subtractions work modulo 2p.
+// Zero tests accept 0 and p.  Values are made canonical when they leave for memory
+// (canon()).
 // ---------------------------------------------------------------------------
-struct FqL {
+
+// 2p as a parameter set: reduce_once and the subtraction of Fp on it work modulo 2p
+template <class P>
+struct TwoP {
+    static constexpr uint32_t P0 = P::P0 << 1, P1 = P::P1 << 1 | P::P0 >> 31, P2 = P::P2 << 1 | P::P1 >> 31,
+                              P3 = P::P3 << 1 | P::P2 >> 31, P4 = P::P4 << 1 | P::P3 >> 31,
+                              P5 = P::P5 << 1 | P::P4 >> 31, P6 = P::P6 << 1 | P::P5 >> 31,
+                              P7 = P::P7 << 1 | P::P6 >> 31;
+};
+
+template <class P>
+struct alignas(32) FpL {
     uint32_t v[8];
-    FqL() = default;
-    __device__ __forceinline__ FqL(const Fq &c)
+    FpL() = default;
+    __device__ __forceinline__ FpL(const Fp<P> &c)
     {
 #pragma unroll
         for (int j = 0; j < 8; ++j) v[j] = c.v[j];
     }
-    __device__ __forceinline__ static FqL zero() { return Fq::zero(); }
-    __device__ __forceinline__ static FqL one() { return Fq::one(); }
+    __device__ __forceinline__ static FpL zero() { return Fp<P>::zero(); }
+    __device__ __forceinline__ static FpL one() { return Fp<P>::one(); }
     __device__ __forceinline__ bool is_zero() const // 0 or p
     {
         uint32_t x = 0, y = 0;
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
             x |= v[j];
-            y |= v[j] ^ mod_word<FqParams>(j);
+            y |= v[j] ^ mod_word<P>(j);
         }
         return x == 0 || y == 0;
     }
-    __device__ __forceinline__ Fq canon() const
+    __device__ __forceinline__ Fp<P> canon() const
     {
-        Fq r;
+        Fp<P> r;
 #pragma unroll
         for (int j = 0; j < 8; ++j) r.v[j] = v[j];
-        reduce_once<FqParams>(r.v);
+        reduce_once<P>(r.v);
         return r;
     }
-    __device__ __forceinline__ bool operator==(const FqL &o) const { return canon() == o.canon(); }
-    __device__ __forceinline__ bool operator!=(const FqL &o) const { return !(*this == o); }
+    __device__ __forceinline__ bool operator==(const FpL &o) const { return canon() == o.canon(); }
+    __device__ __forceinline__ bool operator!=(const FpL &o) const { return !(*this == o); }
 };
+using FqL = FpL<FqParams>;
+using FrL = FpL<FrParams>;
 
-// 2p as a parameter set: reduce_once<TwoP> and the modular additions below
-struct TwoP {
-    static constexpr uint32_t P0 = 0xb0f9fa8eu, P1 = 0x7841182du, P2 = 0xd0e3951au, P3 = 0x2f02d522u,
-                              P4 = 0x0302b0bbu, P5 = 0x70a08b6du, P6 = 0xc2634053u, P7 = 0x60c89ce5u;
-};
-
-__device__ NKR_MUL_ATTR_FN FqL operator*(FqL a, FqL b)
+template <class P>
+__device__ NKR_MUL_ATTR FpL<P> operator*(FpL<P> a, FpL<P> b)
 {
-    FqL r;
-    mont_mul<FqParams>(a.v, b.v, r.v);
+    FpL<P> r;
+    mont_mul<P>(a.v, b.v, r.v);
     return r;
 }
-__device__ __forceinline__ FqL sqr(const FqL &a) { return a * a; }
-__device__ __forceinline__ FqL operator+(const FqL &a, const FqL &b)
+template <class P>
+__device__ __forceinline__ FpL<P> sqr(const FpL<P> &a)
 {
-    FqL r;
+    return a * a;
+}
+template <class P>
+__device__ __forceinline__ FpL<P> operator+(const FpL<P> &a, const FpL<P> &b)
+{
+    FpL<P> r;
     add_words(r.v, a.v, b.v);
-    reduce_once<TwoP>(r.v);
+    reduce_once<TwoP<P>>(r.v);
     return r;
 }
-__device__ __forceinline__ FqL operator-(const FqL &a, const FqL &b)
+template <class P>
+__device__ __forceinline__ FpL<P> operator-(const FpL<P> &a, const FpL<P> &b)
 {
-    Fp<TwoP> x, y;
+    Fp<TwoP<P>> x, y;
 #pragma unroll
     for (int j = 0; j < 8; ++j) x.v[j] = a.v[j], y.v[j] = b.v[j];
     x = x - y;
-    FqL r;
+    FpL<P> r;
 #pragma unroll
     for (int j = 0; j < 8; ++j) r.v[j] = x.v[j];
     return r;
 }
-__device__ __forceinline__ FqL neg(const FqL &a) { return FqL::zero() - a; }
-__device__ __forceinline__ FqL dbl(const FqL &a) { return a + a; }
+template <class P>
+__device__ __forceinline__ FpL<P> neg(const FpL<P> &a)
+{
+    return FpL<P>::zero() - a;
+}
+template <class P>
+__device__ __forceinline__ FpL<P> dbl(const FpL<P> &a)
+{
+    return a + a;
+}
 
 // ---------------------------------------------------------------------------
 // Fq2 = Fq[u] / (u^2 + 1)  (libff alt_bn128_Fq2, non_residue = -1)

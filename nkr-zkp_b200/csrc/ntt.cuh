@@ -60,6 +60,12 @@ int ntt_dif(const NttTables &t, Fr *data, bool inverse, const Fr *pre, const Fr 
 int ntt_dit(const NttTables &t, Fr *data, bool inverse, const Fr *pre, const Fr *post,
             const Fr *post_const, cudaStream_t st);
 
+// DIF transform of data whose last pass writes the result to out in natural order (post is
+// indexed by the transform's own, bit-reversed position); data is used up, out must not
+// overlap it
+int ntt_dif_natural(const NttTables &t, Fr *data, Fr *out, bool inverse, const Fr *pre, const Fr *post,
+                    const Fr *post_const, cudaStream_t st);
+
 // out[bitrev(j)] = in[j] * (scale ? scale[j] : scale_const ? *scale_const : 1)
 int ntt_bitrev_permute(const Fr *in, Fr *out, uint64_t n, const Fr *scale, const Fr *scale_const,
                        cudaStream_t st);

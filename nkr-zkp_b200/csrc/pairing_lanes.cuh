@@ -124,7 +124,7 @@ __device__ __forceinline__ Fq redc_sum(const uint32_t *t)
     Fq r;
     lazy::redc_low(t, lo);
     add_words(r.v, lo, t + 8);
-    reduce_once<TwoP>(r.v);
+    reduce_once<TwoP<FqParams>>(r.v);
     reduce_once<FqParams>(r.v);
     return r;
 }
