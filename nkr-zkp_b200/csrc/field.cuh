@@ -500,10 +500,138 @@ __device__ __forceinline__ Fp<P> mont_mul_cc(const Fp<P> &a, const Fp<P> &b)
     return r;
 }
 
+
+// r = t[0..7] R^-1 mod p (R = 2^256), at most p: the rows of mont_mul without a product
 template <class P>
-__device__ __forceinline__ Fp<P> sqr(const Fp<P> &a)
+__device__ __forceinline__ void redc_low(const uint32_t *t, uint32_t *r)
 {
-    return a * a;
+    uint32_t e[9], o[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) e[j] = t[j], o[j] = 0;
+    e[8] = 0;
+    eo_reduce_row<P>(e, o);
+#pragma unroll
+    for (int i = 1; i < 8; ++i) {
+        uint32_t ne[9], no[8];
+        const uint32_t w = e[1];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) ne[j] = o[j];
+#pragma unroll
+        for (int j = 0; j < 7; ++j) no[j] = e[j + 2];
+        no[7] = 0;
+        const uint32_t m = (ne[0] + w) * P::INV;
+        eo_mad_fit(no, P::P1, P::P3, P::P5, P::P7, m);
+        eo_mad_word(ne, ne[8], w, P::P0, P::P2, P::P4, P::P6, m);
+#pragma unroll
+        for (int j = 0; j < 9; ++j) e[j] = ne[j];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) o[j] = no[j];
+    }
+    add_words(r, e + 1, o);
+}
+
+// x += (a[0], a[2], ..) b, n words of a into adjacent word pairs of x, with the carry
+// added to the word after them
+__device__ __forceinline__ void mad_chain(uint32_t *x, const uint32_t *a, int n, uint32_t b)
+{
+    if (n == 4)
+        eo_mad(x, x[8], a[0], a[2], a[4], a[6], b);
+    else if (n == 3)
+        asm("mad.lo.cc.u32  %0, %7, %10, %0;\n\t"
+            "madc.hi.cc.u32 %1, %7, %10, %1;\n\t"
+            "madc.lo.cc.u32 %2, %8, %10, %2;\n\t"
+            "madc.hi.cc.u32 %3, %8, %10, %3;\n\t"
+            "madc.lo.cc.u32 %4, %9, %10, %4;\n\t"
+            "madc.hi.cc.u32 %5, %9, %10, %5;\n\t"
+            "addc.u32       %6, %6, 0;"
+            : "+&r"(x[0]), "+&r"(x[1]), "+&r"(x[2]), "+&r"(x[3]), "+&r"(x[4]), "+&r"(x[5]), "+&r"(x[6])
+            : "r"(a[0]), "r"(a[2]), "r"(a[4]), "r"(b));
+    else if (n == 2)
+        asm("mad.lo.cc.u32  %0, %5, %7, %0;\n\t"
+            "madc.hi.cc.u32 %1, %5, %7, %1;\n\t"
+            "madc.lo.cc.u32 %2, %6, %7, %2;\n\t"
+            "madc.hi.cc.u32 %3, %6, %7, %3;\n\t"
+            "addc.u32       %4, %4, 0;"
+            : "+&r"(x[0]), "+&r"(x[1]), "+&r"(x[2]), "+&r"(x[3]), "+&r"(x[4])
+            : "r"(a[0]), "r"(a[2]), "r"(b));
+    else if (n == 1)
+        asm("mad.lo.cc.u32  %0, %3, %4, %0;\n\t"
+            "madc.hi.cc.u32 %1, %3, %4, %1;\n\t"
+            "addc.u32       %2, %2, 0;"
+            : "+&r"(x[0]), "+&r"(x[1]), "+&r"(x[2])
+            : "r"(a[0]), "r"(b));
+}
+
+// t = 2 t + sum_i a_i^2 2^(64 i) on 16 words, 2 t < 2^512 and no carry out
+__device__ __forceinline__ void double_add_squares(uint32_t *t, const uint32_t *a)
+{
+#pragma unroll
+    for (int j = 15; j > 0; --j) t[j] = __funnelshift_l(t[j - 1], t[j], 1);
+    t[0] <<= 1;
+    uint32_t c = 0;
+    asm("mad.lo.cc.u32  %0, %9,  %9,  %0;\n\t"
+        "madc.hi.cc.u32 %1, %9,  %9,  %1;\n\t"
+        "madc.lo.cc.u32 %2, %10, %10, %2;\n\t"
+        "madc.hi.cc.u32 %3, %10, %10, %3;\n\t"
+        "madc.lo.cc.u32 %4, %11, %11, %4;\n\t"
+        "madc.hi.cc.u32 %5, %11, %11, %5;\n\t"
+        "madc.lo.cc.u32 %6, %12, %12, %6;\n\t"
+        "madc.hi.cc.u32 %7, %12, %12, %7;\n\t"
+        "addc.u32       %8, 0, 0;"
+        : "+&r"(t[0]), "+&r"(t[1]), "+&r"(t[2]), "+&r"(t[3]), "+&r"(t[4]), "+&r"(t[5]), "+&r"(t[6]), "+&r"(t[7]), "=r"(c)
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]));
+    asm("add.cc.u32     %8, %8,  0xffffffff;\n\t" // carry in
+        "madc.lo.cc.u32 %0, %9,  %9,  %0;\n\t"
+        "madc.hi.cc.u32 %1, %9,  %9,  %1;\n\t"
+        "madc.lo.cc.u32 %2, %10, %10, %2;\n\t"
+        "madc.hi.cc.u32 %3, %10, %10, %3;\n\t"
+        "madc.lo.cc.u32 %4, %11, %11, %4;\n\t"
+        "madc.hi.cc.u32 %5, %11, %11, %5;\n\t"
+        "madc.lo.cc.u32 %6, %12, %12, %6;\n\t"
+        "madc.hi.u32    %7, %12, %12, %7;"
+        : "+&r"(t[8]), "+&r"(t[9]), "+&r"(t[10]), "+&r"(t[11]), "+&r"(t[12]), "+&r"(t[13]), "+&r"(t[14]), "+&r"(t[15]),
+          "+&r"(c)
+        : "r"(a[4]), "r"(a[5]), "r"(a[6]), "r"(a[7]));
+}
+
+// a^2 2^-256 mod p, bounds as mont_mul: the 28 products of distinct words once, doubled,
+// and 8 squares, then the reduction of the low half (100 wide multiply-adds instead of 128)
+template <class P>
+__device__ __forceinline__ void mont_sqr(const uint32_t *a, uint32_t *r)
+{
+    uint32_t e[16], o[16]; // o[k] holds word offset k + 1
+#pragma unroll
+    for (int j = 0; j < 16; ++j) e[j] = o[j] = 0;
+#pragma unroll
+    for (int i = 0; i < 7; ++i) {
+        // a_i a_j, j > i: offsets i + j odd into o, even into e; chains from the lowest
+        mad_chain(o + 2 * i, a + i + 1, (8 - i) / 2, a[i]);
+        mad_chain(e + 2 * i + 2, a + i + 2, (7 - i) / 2, a[i]);
+    }
+    uint32_t t[16], c = 0;
+    t[0] = 0;
+    uint32_t hi[8];
+    add_words_carry(t + 1, e + 1, o, c);
+    uint32_t eh[8];
+#pragma unroll
+    for (int j = 0; j < 7; ++j) eh[j] = e[9 + j];
+    eh[7] = 0;
+    add_words_carry(hi, eh, o + 8, c);
+#pragma unroll
+    for (int j = 0; j < 7; ++j) t[9 + j] = hi[j];
+    double_add_squares(t, a);
+    uint32_t lo[8];
+    redc_low<P>(t, lo);
+    add_words(r, lo, t + 8);
+}
+
+template <class P>
+__device__ NKR_MUL_ATTR Fp<P> sqr(Fp<P> a)
+{
+    Fp<P> r;
+    mont_sqr<P>(a.v, r.v);
+    reduce_once<P>(r.v);
+    return r;
 }
 
 // Montgomery -> canonical integer (same limb layout)
@@ -561,6 +689,48 @@ struct TwoP {
                               P7 = P::P7 << 1 | P::P6 >> 31;
 };
 
+// (a b + c d) 2^-256 mod p with one reduction: for inputs below 2p the running value stays
+// below 2^32 (a + c + p) <= 2^32 5p < 2^288 and the result below 2.51 p; one conditional
+// subtraction of 2p brings it below 2p (192 wide multiply-adds instead of 256)
+template <class P>
+__device__ __forceinline__ void mont_mul_add(const uint32_t *a, const uint32_t *b, const uint32_t *x,
+                                             const uint32_t *y, uint32_t *r)
+{
+    uint32_t e[9], o[8];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const uint64_t u = uint64_t(a[2 * j]) * b[0], w = uint64_t(a[2 * j + 1]) * b[0];
+        e[2 * j] = uint32_t(u);
+        e[2 * j + 1] = uint32_t(u >> 32);
+        o[2 * j] = uint32_t(w);
+        o[2 * j + 1] = uint32_t(w >> 32);
+    }
+    e[8] = 0;
+    eo_mad_fit(o, x[1], x[3], x[5], x[7], y[0]);
+    eo_mad(e, e[8], x[0], x[2], x[4], x[6], y[0]);
+    eo_reduce_row<P>(e, o);
+#pragma unroll
+    for (int i = 1; i < 8; ++i) {
+        uint32_t ne[9], no[8];
+        const uint32_t w = e[1];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) ne[j] = o[j];
+#pragma unroll
+        for (int j = 0; j < 7; ++j) no[j] = e[j + 2];
+        no[7] = 0;
+        eo_mad_fit(no, a[1], a[3], a[5], a[7], b[i]);
+        eo_mad_word(ne, ne[8], w, a[0], a[2], a[4], a[6], b[i]);
+        eo_mad_fit(no, x[1], x[3], x[5], x[7], y[i]);
+        eo_mad(ne, ne[8], x[0], x[2], x[4], x[6], y[i]);
+        eo_reduce_row<P>(ne, no);
+#pragma unroll
+        for (int j = 0; j < 9; ++j) e[j] = ne[j];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) o[j] = no[j];
+    }
+    add_words(r, e + 1, o);
+}
+
 template <class P>
 struct alignas(32) FpL {
     uint32_t v[8];
@@ -604,9 +774,20 @@ __device__ NKR_MUL_ATTR FpL<P> operator*(FpL<P> a, FpL<P> b)
     return r;
 }
 template <class P>
-__device__ __forceinline__ FpL<P> sqr(const FpL<P> &a)
+__device__ NKR_MUL_ATTR FpL<P> sqr(FpL<P> a)
 {
-    return a * a;
+    FpL<P> r;
+    mont_sqr<P>(a.v, r.v);
+    return r;
+}
+// a b + c d
+template <class P>
+__device__ NKR_MUL_ATTR FpL<P> mul_add(FpL<P> a, FpL<P> b, FpL<P> c, FpL<P> d)
+{
+    FpL<P> r;
+    mont_mul_add<P>(a.v, b.v, c.v, d.v, r.v);
+    reduce_once<TwoP<P>>(r.v);
+    return r;
 }
 template <class P>
 __device__ __forceinline__ FpL<P> operator+(const FpL<P> &a, const FpL<P> &b)
@@ -710,41 +891,13 @@ __device__ __forceinline__ void mul_wide(const uint32_t *a, const uint32_t *b, u
     for (int j = 0; j < 7; ++j) t[9 + j] = hi[j];
 }
 
-// r = t[0..7] R^-1 mod p (R = 2^256), at most p: the rows of mont_mul without a product
-__device__ __forceinline__ void redc_low(const uint32_t *t, uint32_t *r)
-{
-    uint32_t e[9], o[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) e[j] = t[j], o[j] = 0;
-    e[8] = 0;
-    eo_reduce_row<FqParams>(e, o);
-#pragma unroll
-    for (int i = 1; i < 8; ++i) {
-        uint32_t ne[9], no[8];
-        const uint32_t w = e[1];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) ne[j] = o[j];
-#pragma unroll
-        for (int j = 0; j < 7; ++j) no[j] = e[j + 2];
-        no[7] = 0;
-        const uint32_t m = (ne[0] + w) * FqParams::INV;
-        eo_mad_fit(no, FqParams::P1, FqParams::P3, FqParams::P5, FqParams::P7, m);
-        eo_mad_word(ne, ne[8], w, FqParams::P0, FqParams::P2, FqParams::P4, FqParams::P6, m);
-#pragma unroll
-        for (int j = 0; j < 9; ++j) e[j] = ne[j];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) o[j] = no[j];
-    }
-    add_words(r, e + 1, o);
-}
-
 // Montgomery reduction T R^-1 mod p of a 512-bit T < p R: the low half's reduction and the
 // high half, below 2p before the conditional subtraction
 __device__ __forceinline__ Fq redc_wide(const uint32_t *t)
 {
     Fq r;
     uint32_t lo[8];
-    redc_low(t, lo);
+    redc_low<FqParams>(t, lo);
     add_words(r.v, lo, t + 8);
     reduce_once<FqParams>(r.v);
     return r;
@@ -841,6 +994,36 @@ __device__ NKR_MUL_ATTR_FN Fq2L operator*(Fq2L a, Fq2L b)
     return r;
 }
 
+
+// Fq2 on coordinates below 2p, the compute type of the G2 accumulation: each coordinate of a
+// product is a sum of two products with one reduction (mul_add), 384 wide multiply-adds
+// like three separate products, without the additions and conditional subtractions of
+// Karatsuba's form and with half its live values
+struct Fq2M {
+    FqL c0, c1;
+    Fq2M() = default;
+    __device__ __forceinline__ Fq2M(const FqL &a, const FqL &b) : c0(a), c1(b) {}
+    __device__ __forceinline__ Fq2M(const Fq2 &a) : c0(a.c0), c1(a.c1) {}
+    __device__ __forceinline__ static Fq2M zero() { return Fq2::zero(); }
+    __device__ __forceinline__ static Fq2M one() { return Fq2::one(); }
+    __device__ __forceinline__ bool is_zero() const { return c0.is_zero() && c1.is_zero(); }
+    __device__ __forceinline__ Fq2 canon() const { return {c0.canon(), c1.canon()}; }
+    __device__ __forceinline__ bool operator==(const Fq2M &o) const { return c0 == o.c0 && c1 == o.c1; }
+};
+__device__ __forceinline__ Fq2M operator+(const Fq2M &a, const Fq2M &b) { return {a.c0 + b.c0, a.c1 + b.c1}; }
+__device__ __forceinline__ Fq2M operator-(const Fq2M &a, const Fq2M &b) { return {a.c0 - b.c0, a.c1 - b.c1}; }
+__device__ __forceinline__ Fq2M neg(const Fq2M &a) { return {neg(a.c0), neg(a.c1)}; }
+__device__ __forceinline__ Fq2M dbl(const Fq2M &a) { return {dbl(a.c0), dbl(a.c1)}; }
+__device__ __forceinline__ Fq2M operator*(const Fq2M &a, const Fq2M &b)
+{
+    const FqL x = mul_add(a.c0, b.c0, neg(a.c1), b.c1);
+    return {x, mul_add(a.c0, b.c1, a.c1, b.c0)};
+}
+__device__ __forceinline__ Fq2M sqr(const Fq2M &a)
+{
+    const FqL x = (a.c0 + a.c1) * (a.c0 - a.c1);
+    return {x, dbl(a.c0 * a.c1)};
+}
 
 __device__ inline Fq2 inverse(const Fq2 &a)
 {

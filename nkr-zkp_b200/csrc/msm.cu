@@ -138,7 +138,7 @@ struct MsmArith<Fq> {
 };
 template <>
 struct MsmArith<Fq2> {
-    using type = Fq2;
+    using type = Fq2M;
     using quad = Fq2L;
 };
 template <class F>
@@ -148,6 +148,7 @@ using QF = typename MsmArith<F>::quad;
 
 __device__ __forceinline__ Fq msm_out(const FqL &x) { return x.canon(); }
 __device__ __forceinline__ Fq2 msm_out(const Fq2 &x) { return x; }
+__device__ __forceinline__ Fq2 msm_out(const Fq2M &x) { return x.canon(); }
 
 template <class C>
 __device__ __forceinline__ auto stx(const Xyzz<C> &c) -> Xyzz<decltype(msm_out(c.x))>
@@ -282,11 +283,11 @@ struct SmXyzzFq {
 // G2: Fq2 coordinates (16 x 32-bit words), the library's Montgomery domain.
 template <int BS>
 struct SmXyzzFq2 {
-    using point = Affine<Fq2>;
+    using point = Affine<Fq2M>;
     uint32_t *s; // the block's area + threadIdx.x; 64 words per thread
-    __device__ __forceinline__ Fq2 ld(int f) const
+    __device__ __forceinline__ Fq2M ld(int f) const
     {
-        Fq2 v;
+        Fq2M v;
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
             v.c0.v[j] = s[(f * 16 + j) * BS];
@@ -294,7 +295,7 @@ struct SmXyzzFq2 {
         }
         return v;
     }
-    __device__ __forceinline__ void st(int f, const Fq2 &v) const
+    __device__ __forceinline__ void st(int f, const Fq2M &v) const
     {
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
@@ -302,19 +303,35 @@ struct SmXyzzFq2 {
             s[(f * 16 + 8 + j) * BS] = v.c1.v[j];
         }
     }
-    __device__ __forceinline__ void set(const Xyzz<Fq2> &a) const
+    __device__ __forceinline__ void set(const Xyzz<Fq2M> &a) const
     {
         st(0, a.x);
         st(1, a.y);
         st(2, a.zz);
         st(3, a.zzz);
     }
-    __device__ __forceinline__ Xyzz<Fq2> out() const { return {ld(0), ld(1), ld(2), ld(3)}; }
-    __device__ __forceinline__ static point load(const Affine<Fq2> &p) { return p; }
+    __device__ __forceinline__ Xyzz<Fq2> out() const { return stx(Xyzz<Fq2M>{ld(0), ld(1), ld(2), ld(3)}); }
+    __device__ __forceinline__ static point load(const Affine<Fq2> &p) { return lda(p); }
 };
 
+// a b - c d
+__device__ __forceinline__ FqL mul_sub(const FqL &a, const FqL &b, const FqL &c, const FqL &d)
+{
+    return mul_add(a, b, neg(c), d); // one reduction for both products
+}
+__device__ __forceinline__ Fq2M mul_sub(const Fq2M &a, const Fq2M &b, const Fq2M &c, const Fq2M &d)
+{
+    const Fq2M cd = c * d;
+    return a * b - cd;
+}
+
 // acc + q (madd-2008-s: 8M + 2S) on a shared-memory accumulator, q may be infinity;
-// each product comes right before its first use, which keeps few values live
+// each product comes right before its first use, which keeps few values live.  Bound by the
+// multiply pipe, so the squarings (100 wide multiply-adds) and the last coordinate's two
+// products with one reduction (192) bring G1's 1,280 down to 1,160: the 2^20 MSM 3.91 ->
+// 3.64 ms.  G2 in Fq2M instead of three reduced products per Fq2 product: 100,001 points
+// 1.97 -> 1.84 ms, the 2^20 prove 10.0 -> 9.7 ms; in Fq2L (two reductions, 320 instead of
+// 384 per product, but more live values and spills) 1.94 ms and 10.0 ms.
 template <class Acc, class C>
 __device__ __forceinline__ void sm_add_affine(const Acc &a, const Affine<C> &q)
 {
@@ -336,8 +353,7 @@ __device__ __forceinline__ void sm_add_affine(const Acc &a, const Affine<C> &q)
     const C qq = a.ld(0) * pp;
     const C ox = sqr(r) - ppp - dbl(qq);
     a.st(0, ox);
-    const C y1ppp = a.ld(1) * ppp;
-    a.st(1, r * (qq - ox) - y1ppp);
+    a.st(1, mul_sub(r, qq - ox, a.ld(1), ppp));
     a.st(2, a.ld(2) * pp);
 }
 
@@ -396,7 +412,8 @@ __device__ __forceinline__ void acc_l1_body(const uint32_t *__restrict__ offsets
             bend = offsets[b + 1];
         }
         const uint32_t e = entries[j];
-        typename Acc::point p = Acc::load(pts[e & 0x7fffffffu]);
+        const Affine<F> base = pts[e & 0x7fffffffu]; // whole: 16-byte vector loads
+        typename Acc::point p = Acc::load(base);
         if (e >> 31) p = affine_neg(p);
         sm_add_affine(acc, p);
     }

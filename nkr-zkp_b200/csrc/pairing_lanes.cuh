@@ -122,7 +122,7 @@ __device__ __forceinline__ Fq redc_sum(const uint32_t *t)
 {
     uint32_t lo[8];
     Fq r;
-    lazy::redc_low(t, lo);
+    redc_low<FqParams>(t, lo);
     add_words(r.v, lo, t + 8);
     reduce_once<TwoP<FqParams>>(r.v);
     reduce_once<FqParams>(r.v);

@@ -55,6 +55,8 @@ def test_products_of_extreme_words(ctx, field, mod):
     want = np.stack([O.int_to_limbs(x * y * rinv % mod) for x in vals for y in vals])
     if field != 2:
         assert np.array_equal(ctx.field_op(field, 0, a, b), want)
+        squares = np.stack([O.int_to_limbs(x * x * rinv % mod) for x in vals])
+        assert np.array_equal(ctx.field_op(field, 3, limbs), squares)
         return
     # Fq2: (x + y u)(y + x u) = (x^2 + y^2) u and (x + y u)(x - y u) = x^2 + y^2
     sq = np.stack([O.int_to_limbs((x * x + y * y) * rinv % mod) for x in vals for y in vals])
