@@ -48,17 +48,26 @@
 
 namespace nkr {
 
-// Entries per level-1 segment (mixed additions per thread) of an MSM of `total` entries:
-// enough segments for one and a half warps per scheduler (148 x 4 x 48 threads), where an
-// addition still runs at its own latency, within kSegMin..kmax entries.  The count is
-// known on the device only (zero digits and class members have no entry), so every
-// kernel that needs the length computes it from the sort's total.
+// Entries per level-1 segment (mixed additions per thread) of an MSM of `total` entries.
+// Up to 32 per segment of one and a half warps per scheduler (148 x 4 x 48 threads), where
+// an addition still runs at its own latency, there are that many segments of at least
+// kSegMin entries.  Beyond, the segments (at most kmax entries) make whole waves of the
+// resident threads.  The count is known on the device only (zero digits and class members
+// have no entry), so every kernel that needs the length computes it from the sort's total.
 constexpr uint32_t kSegMin = 4;
 constexpr uint32_t kSegSpread = 148 * 4 * 48;
-__host__ __device__ __forceinline__ uint32_t seg_len(uint32_t total, uint32_t kmax)
+__host__ __device__ constexpr uint32_t level1_resident(int group) // threads of the level-1 kernel
 {
-    const uint32_t k = (total + kSegSpread - 1) / kSegSpread;
-    return k < kSegMin ? kSegMin : k > kmax ? kmax : k;
+    return group == 1 ? 148 * 4 * 128 : 148 * 3 * 128;
+}
+__host__ __device__ __forceinline__ uint32_t seg_len(uint32_t total, uint32_t kmax, int group)
+{
+    if (total <= kSegSpread * kmax) {
+        const uint32_t k = (total + kSegSpread - 1) / kSegSpread;
+        return k < kSegMin ? kSegMin : k;
+    }
+    const uint64_t res = level1_resident(group), waves = (total + res * kmax - 1) / (res * kmax);
+    return uint32_t((total + res * waves - 1) / (res * waves));
 }
 
 struct MsmShape {
@@ -69,13 +78,22 @@ struct MsmShape {
     uint32_t B = 0;  // buckets per set: 2^(c-1)
     uint32_t nb = 0; // total buckets: folded ? B : W * B
     int k1 = 32;     // most entries per level-1 segment (seg_len)
+    // buckets of at most this many level-1 pieces are summed where they are consumed, larger
+    // ones go through the fix-up levels first
+    uint32_t small_pieces = 4;
     uint64_t entries_max() const { return uint64_t(W) * n; }
     // most segments over all entry counts up to entries_max
     uint64_t segments_max() const
     {
-        const uint64_t e = entries_max(), fine = (e + kSegMin - 1) / kSegMin, coarse = (e + k1 - 1) / k1;
-        const uint64_t spread = fine < kSegSpread ? fine : kSegSpread;
-        return coarse > spread ? coarse : spread;
+        const uint64_t e = entries_max(), fine = (e + kSegMin - 1) / kSegMin;
+        if (e <= uint64_t(kSegSpread) * k1) return fine < kSegSpread ? fine : kSegSpread;
+        // (either group: a shape does not know its own)
+        uint64_t most = 0;
+        for (int g = 1; g <= 2; ++g) {
+            const uint64_t res = level1_resident(g), segs = (e + res * k1 - 1) / (res * k1) * res;
+            most = most > segs ? most : segs;
+        }
+        return most;
     }
     bool same_sort(const MsmShape &o) const
     {
@@ -84,6 +102,10 @@ struct MsmShape {
 };
 
 MsmShape msm_shape(uint64_t n, bool folded, int group, int c_override = 0);
+// Field products of a folded MSM of n points with c-bit windows: n ceil(255 / c) mixed
+// additions (10 products each) for the accumulation and about two full additions per bucket
+// for the reduction (16 products' time each on a quad, at half of level 1's rate).
+double msm_work(uint64_t n, int c);
 
 // Digit sort of one scalar vector: bucket offsets and entries in bucket order.
 struct MsmSort {

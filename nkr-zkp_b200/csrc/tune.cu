@@ -10,6 +10,8 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <utility>
+#include <vector>
 
 #include "msm.cuh"
 #include "prover.cuh"
@@ -100,6 +102,7 @@ int measure(nkr_b200_ctx *ctx, int lg)
     const int c0 = msm_shape(n, true, 1).c;
     int best_c = c0;
     float best = 1e30f;
+    std::vector<std::pair<int, float>> times;
     int status = NKR_B200_OK;
     for (int c = c0 - 3; c <= c0 + 1 && status == NKR_B200_OK; ++c) {
         if (c < 6 || c > 22) continue;
@@ -122,8 +125,17 @@ int measure(nkr_b200_ctx *ctx, int lg)
             cudaEventElapsedTime(&ms, e0, e1);
             if (rep > 0 && ms < t_min) t_min = ms; // rep 0 warms up
         }
-        if (t_min < best) {
-            best = t_min;
+        times.push_back({c, t_min});
+        if (t_min < best) best = t_min;
+    }
+    // Widths within 3% of the fastest alone differ in the work that they leave for others:
+    // of these the one of the least work is kept (a batch of 8 proofs of 2^15 constraints
+    // took 7.0 to 7.7 ms with whichever happened to be the fastest)
+    double least = 1e300;
+    for (const auto &[c, t] : times) {
+        const double work = msm_work(n, c);
+        if (t <= 1.03f * best && work < least) {
+            least = work;
             best_c = c;
         }
     }
