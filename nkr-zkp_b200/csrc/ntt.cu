@@ -244,10 +244,12 @@ __global__ void k_quotient(const Fr *a, const Fr *b, const Fr *c, Fr *h, uint64_
 }
 
 // pass split: at most max_stages radix-2 stages per pass, spread evenly
-// (ts holds up to 8 passes: max_stages >= 4 for logn <= 28)
+// (ts holds up to 8 passes: max_stages >= 4 for logn <= 28).  A single pass is a single
+// block, whose SM is busy with the products alone from 2^9 on: 2^10 takes 23.6 us in one
+// pass and 13.9 us in two, 2^8 10.3 and 12.3 us.
 int pass_plan(int logn, int max_stages, int *ts)
 {
-    const int np = (logn + max_stages - 1) / max_stages;
+    const int np = std::max((logn + max_stages - 1) / max_stages, logn >= 9 ? 2 : 1);
     for (int i = 0; i < np; ++i) ts[i] = logn / np + (i < logn % np ? 1 : 0);
     return np;
 }
