@@ -15,8 +15,8 @@ of a fresh seeded witness on resident keys.
   e2e       the same through the C ABI from pinned host memory: witness upload,
             prove, raw-proof download, blinding with seeded r, s, proof download.
   roofline  the dominant kernel (MSM bucket accumulation) in Fq-multiplications/s
-            against the instruction-issue ceiling of the product (SMs x 4 warp
-            instructions per cycle x 32 lanes x SM clock / instructions per
+            against the rate at which the multiply pipe takes its wide
+            multiply-adds (SMs x 32 lanes x SM clock / multiply-adds per
             product); HBM bytes of the same kernel against the measured copy
             bandwidth beside it.
   cpu_baseline  one single-threaded prove of the same circuit, key and witness by
@@ -56,21 +56,20 @@ METRIC = "Groth16 prove ms @2^20 constraints (bit-exact)"
 # DRAM read + write bytes per (point, digit) entry of the G1 accumulation kernel,
 # from an ncu capture at 2^18 points (a 2^20 capture would hold ~6 GB of keys on
 # the device); traffic grows with entries (one random base gather per entry)
-TRAFFIC_PER_ENTRY = (439.882752e6 + 20.989440e6) / 3932125   # 117.2 B per entry
-TRAFFIC_SOURCE = ("ncu dram__bytes_read.sum + dram__bytes_write.sum of k_acc_l1_g1 on the "
-                  "2^18-point uniform G1 MSM of --mode kernels (3,932,125 entries), 117.2 B "
+TRAFFIC_PER_ENTRY = (443.377152e6 + 23.237632e6) / 3932126   # 118.7 B per entry
+TRAFFIC_SOURCE = ("ncu dram__bytes_read.sum + dram__bytes_write.sum of k_acc_l1_g1 on a "
+                  "2^18-point uniform G1 MSM with 17-bit windows (3,932,126 entries), 118.7 B "
                   "per entry, scaled by this launch's entries")
-# Thread instructions per 52-bit-limb Fq product in the lazily reduced form the G1
-# accumulation runs: ncu smsp__inst_executed.sum x 32 over the products of
-# nkr_b200_bench_mul's variant 4 (6,603,139,584 warp instructions for
-# 148 x 16 x 256 threads x 256 x 4 = 620,756,992 products).
-INSTR_PER_PRODUCT = 6603139584 * 32 / 620756992   # 340.4
+# Wide (32 x 32 -> 64-bit) multiply-adds of a mixed addition, per one of its 10 products:
+# 6 products of 128, 2 squarings of 100 and two products with one reduction, 192.  The
+# multiply pipe takes one of them every 4 cycles per warp and scheduler: 32 lanes per SM
+# and cycle.
+WIDE_PER_PRODUCT = (6 * 128 + 2 * 100 + 192) / 10   # 116
+WIDE_LANES_PER_SM = 32
 # Pipe counters of k_acc_l1_g1 from one ncu launch (2^18-point uniform G1 MSM of
 # --mode kernels; profiles/k_acc_l1_g1_msm_2_18.md); percentages of peak.
-ACC_NCU = {"issue_active_pct": 59.27, "fp64_pipe_pct": 40.11, "alu_pipe_pct": 56.05,
-           "fmaheavy_pipe_pct": 18.69, "warps_active_per_sm": 10.68, "registers": 168,
-           "stall_per_issue": {"wait": 0.75, "not_selected": 0.75, "math_pipe_throttle": 0.66,
-                               "long_scoreboard": 0.55},
+ACC_NCU = {"issue_active_pct": 37.85, "fmaheavy_pipe_pct": 84.76, "alu_pipe_pct": 21.15,
+           "warps_active_per_sm": 16.12, "registers": 96,
            "source": "ncu --metrics ... -k regex:k_acc_l1_g1 -c 1, --clock-control none"}
 
 
@@ -474,17 +473,15 @@ def run_b200(args):
 
     # ---- roofline of the dominant kernel (MSM bucket accumulation) ---------------
     peaks = _measured_peaks()
-    # The product roof is the instruction-issue ceiling of the 52-bit-limb Fq product
-    # the G1 accumulation runs: every SM issues 4 warp instructions per cycle and one
-    # product costs INSTR_PER_PRODUCT thread instructions (ncu), so no kernel built
-    # from these products exceeds SMs x 4 x 32 x f_sm / INSTR_PER_PRODUCT products/s.
-    # The best register-resident microbenchmark of the same product (itself at ~60%
-    # issue) is reported beside it.
+    # The product roof is the rate of the multiply pipe, which the accumulation's products
+    # saturate first (ncu: 85% busy): no kernel of these products exceeds
+    # SMs x 32 x f_sm / WIDE_PER_PRODUCT products/s.  The best register-resident
+    # microbenchmark of a product is reported beside it.
     peak_int, _ = ctx.bench_mul(1)
     peak_fp64, _ = ctx.bench_mul(1 | (4 << 8))  # the lazily reduced FP64 form
     sms = torch.cuda.get_device_properties(device).multi_processor_count
     f_sm = (clk.get("sm_mhz") or clk.get("sm_max_mhz") or 1965.0) * 1e6
-    issue_peak = sms * 4 * 32 * f_sm / INSTR_PER_PRODUCT
+    pipe_peak = sms * WIDE_LANES_PER_SM * f_sm / WIDE_PER_PRODUCT
     mb = nk.MsmBases(ctx, 1, be._keep["a_query"]) if hasattr(be, "_keep") and be._keep else None
     roof = None
     if mb is not None:
@@ -505,18 +502,16 @@ def run_b200(args):
         traffic = round(st["entries"] * TRAFFIC_PER_ENTRY) if TRAFFIC_PER_ENTRY else None
         roof = {"bound": "int", "kernel": "k_acc_l1_g1 (G1 bucket accumulation; operator-level MSM "
                                           "over the A query and the workload's witness, no class path)",
-                "achieved": round(achieved / 1e9, 2), "peak": round(issue_peak / 1e9, 2),
-                "unit": "G Fq-mul/s", "frac": round(achieved / issue_peak, 3),
-                "peak_source": f"instruction-issue ceiling of the FP64-limb Fq product: {sms} SMs "
-                               f"x 4 warp instructions/cycle x 32 x {f_sm / 1e6:.0f} MHz (SM clock "
-                               f"sampled in the timed region) / {INSTR_PER_PRODUCT:.1f} instructions "
-                               f"per product (ncu on nkr_b200_bench_mul); no FLOP or integer peak "
-                               f"in MEASURED_PEAKS.json applies",
-                "microbench": {"int_cios": round(peak_int / 1e9, 2),
+                "achieved": round(achieved / 1e9, 2), "peak": round(pipe_peak / 1e9, 2),
+                "unit": "G Fq-mul/s", "frac": round(achieved / pipe_peak, 3),
+                "peak_source": f"multiply-pipe ceiling of the accumulation's products: {sms} SMs "
+                               f"x {WIDE_LANES_PER_SM} wide multiply-adds/cycle x {f_sm / 1e6:.0f} MHz (SM clock "
+                               f"sampled in the timed region) / {WIDE_PER_PRODUCT:.0f} per product; no FLOP or "
+                               f"integer peak in MEASURED_PEAKS.json applies",
+                "microbench": {"int_even_odd": round(peak_int / 1e9, 2),
                                "fp64_52bit": round(peak_fp64 / 1e9, 2),
                                "frac_of_best": round(achieved / max(peak_int, peak_fp64), 3),
-                               "note": "register-resident product chains (nkr_b200_bench_mul), "
-                                       "issue active ~60% themselves"},
+                               "note": "register-resident product chains (nkr_b200_bench_mul)"},
                 "ncu": ACC_NCU,
                 "units_per_launch": {"entries": st["entries"], "fq_muls": muls,
                                      "window_bits": st["window_bits"], "windows": st["windows"],
@@ -563,8 +558,7 @@ def run_b200(args):
         "steps": args.steps, "warmup": args.warmup,
         "ms_per_step": round(wall * 1e3 / args.steps, 3), "higher_is_better": False,
         "scaling": "weak", "vs_baseline": None, "dtype": DTYPE,
-        "arith": "Fr and Fq in 8 x 32-bit limbs on the integer pipe; the G1 MSMs' Fq in "
-                 "5 x 52-bit limbs on the FP64 pipe",
+        "arith": "Fr and Fq in 8 x 32-bit limbs on the integer multiply pipe",
         "data": "synthetic (seeded circuit, witness and toxic waste)",
         "config": _config(kind, param, dens, r1.rows, r1.cols, world),
         "key_device_gib": round(key_gb, 2),
@@ -680,7 +674,7 @@ def run_batch(args):
     line = {
         "metric": "batched Groth16 proofs/s, 64 uneven proofs (bit-exact)", "value": round(bat_pps, 2),
         "unit": "proofs/s", "n_gpus": 1, "steps": args.steps, "warmup": args.warmup,
-        "higher_is_better": True, "dtype": "bn254 (exact modular; u32 limbs, G1 MSM in 52-bit FP64 limbs)",
+        "higher_is_better": True, "dtype": "bn254 (exact modular; u32 limbs)",
         "data": "synthetic (seeded circuits, witnesses and toxic waste)",
         "config": {"workload": "64 proofs: matmul s in [16, 64] or poseidon count 2^6..2^11, "
                                "hybrid density, seed 4", "domains": dict(sorted(hist.items())),
