@@ -542,7 +542,7 @@ __global__ void __launch_bounds__(128) k_fix_up(const uint32_t *__restrict__ off
         const uint32_t off_b = offsets[b];
         const Pieces pc = bucket_pieces(offsets, b, k1);
         uint64_t stride = 1; // pieces between two inputs of this level
-        for (uint32_t level = 1;; ++level, stride *= kFixGroup) {
+        for (uint32_t level = 1; level <= 16; ++level, stride *= kFixGroup) { // 4^16 pieces at most
             const uint64_t beg = uint64_t(g) * kFixGroup * stride;
             C acc = quad_inf<C>();
             for (uint32_t m = 0; m < kFixGroup; ++m) {
@@ -551,7 +551,7 @@ __global__ void __launch_bounds__(128) k_fix_up(const uint32_t *__restrict__ off
                 acc = quad_add(acc, quad_ld(&partials[pc.slot(off_b, k1, uint32_t(idx))]));
             }
             const uint32_t groups = uint32_t((pc.count + kFixGroup * stride - 1) / (kFixGroup * stride));
-            if (groups == 1) {
+            if (groups <= 1) {
                 quad_st(&buckets[b], acc);
                 break;
             }

@@ -198,9 +198,13 @@ __device__ __forceinline__ constexpr uint64_t terms(int t0, int t1 = 0, int t2 =
     return lane_bytes(t0, t1, t2, t3, 0, 0);
 }
 
-// z in signed odd digits (width-4 non-adjacent form), 4 bits a digit
-constexpr uint64_t kZDigits[4] = {0x50000f0001ull, 0x100005000070009ull, 0x300005000b000d00ull, 0x10000050000d000ull};
-constexpr int z_digit(int b) { return (int(kZDigits[b >> 4] >> (4 * (b & 15)) & 15u) ^ 8) - 8; }
+// Digit b of z in signed odd digits (width-4 non-adjacent form, 4 bits a digit).  The table
+// is local: device code cannot index a host constant of namespace scope at run time.
+__host__ __device__ constexpr int z_digit(int b)
+{
+    const uint64_t w[4] = {0x50000f0001ull, 0x100005000070009ull, 0x300005000b000d00ull, 0x10000050000d000ull};
+    return (int(w[b >> 4] >> (4 * (b & 15)) & 15u) ^ 8) - 8;
+}
 constexpr uint64_t z_of_digits()
 {
     uint64_t z = 0;
