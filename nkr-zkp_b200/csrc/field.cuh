@@ -424,7 +424,9 @@ __device__ __forceinline__ void eo_reduce_row(uint32_t *e, uint32_t *o)
 
 // a b 2^-256 mod p, below a b / 2^256 + p and not reduced further: for inputs
 // below 2p the result is below 1.76 p.  The running value stays below
-// 2^32 (a + p), within nine words for a < 2p.
+// 2^32 (a + p), within nine words for a < 2^256 - p; b may be any eight words (with a < p the
+// result is below 2p then).  So a value that a caller hands in, which need not be reduced,
+// goes second.
 template <class P>
 __device__ __forceinline__ void mont_mul(const uint32_t *a, const uint32_t *b, uint32_t *r)
 {
@@ -634,7 +636,7 @@ __device__ NKR_MUL_ATTR Fp<P> sqr(Fp<P> a)
     return r;
 }
 
-// Montgomery -> canonical integer (same limb layout)
+// Montgomery -> canonical integer (same limb layout); any eight words
 template <class P>
 __device__ __forceinline__ Fp<P> from_mont(const Fp<P> &a)
 {
@@ -642,14 +644,29 @@ __device__ __forceinline__ Fp<P> from_mont(const Fp<P> &a)
     one.v[0] = 1;
 #pragma unroll
     for (int i = 1; i < 8; ++i) one.v[i] = 0;
-    return a * one;
+    return a * one; // (one's single word keeps the running value within nine words)
 }
 
-// canonical integer (< p) -> Montgomery
+// integer (any eight words) -> Montgomery
 template <class P>
 __device__ __forceinline__ Fp<P> to_mont(const Fp<P> &a)
 {
-    return a * Fp<P>::r2();
+    return Fp<P>::r2() * a;
+}
+
+// the value below p congruent to eight words that a caller handed in
+template <class P>
+__device__ __forceinline__ Fp<P> reduced(const Fp<P> &a)
+{
+    return Fp<P>::one() * a;
+}
+
+// a b where either of them may be any eight words and the other one is below p
+template <class P>
+__device__ __forceinline__ Fp<P> mul_any(Fp<P> a, const Fp<P> &b)
+{
+    reduce_once<P>(a.v); // below 2^256 - p
+    return a * b;
 }
 
 // a^e for a small public exponent given as 8 limbs (left-to-right square-and-multiply)
@@ -844,6 +861,7 @@ __device__ __forceinline__ Fq2 operator-(const Fq2 &a, const Fq2 &b)
     return {a.c0 - b.c0, a.c1 - b.c1};
 }
 __device__ __forceinline__ Fq2 neg(const Fq2 &a) { return {neg(a.c0), neg(a.c1)}; }
+__device__ __forceinline__ Fq2 reduced(const Fq2 &a) { return {reduced(a.c0), reduced(a.c1)}; }
 __device__ __forceinline__ Fq2 dbl(const Fq2 &a) { return {dbl(a.c0), dbl(a.c1)}; }
 
 // Karatsuba with 3 Montgomery products (one three-product call measured slower:

@@ -833,7 +833,7 @@ __global__ void k_jac_to_affine(const F *__restrict__ jac, Affine<F> *__restrict
         const F zi = inv * pre[j];
         inv = inv * z;
         const F zi2 = sqr(zi);
-        out[i] = {jac[3 * i] * zi2, jac[3 * i + 1] * (zi2 * zi)};
+        out[i] = {zi2 * jac[3 * i], (zi2 * zi) * jac[3 * i + 1]}; // coordinates need not be reduced
     }
 }
 

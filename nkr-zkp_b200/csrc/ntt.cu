@@ -129,7 +129,7 @@ __device__ __forceinline__ void ntt_pass_tile(Fr *sm, Fr *data, int s_lo, int t,
     for (int m = threadIdx.x; m < G; m += blockDim.x) {
         const uint64_t j = base + (uint64_t(m) << s_lo);
         FrL x = in(&data[j]);
-        if (pre) x = x * in(&pre[j]);
+        if (pre) x = in(&pre[j]) * x; // a caller's vector need not be reduced
         put(m, x);
     }
     __syncthreads();
@@ -224,23 +224,23 @@ __global__ void k_bitrev_permute(const Fr *in, Fr *out, int logn, const Fr *scal
     if (j >= n) return;
     Fr x = in[j];
     if (scale)
-        x = x * scale[j];
+        x = scale[j] * x;
     else if (scale_const)
-        x = x * *scale_const;
+        x = *scale_const * x;
     out[brev_n(uint32_t(j), logn)] = x;
 }
 
 __global__ void k_scale_const(Fr *d, uint64_t n, const Fr *c)
 {
     const uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i < n) d[i] = d[i] * *c;
+    if (i < n) d[i] = *c * d[i];
 }
 
 __global__ void k_quotient(const Fr *a, const Fr *b, const Fr *c, Fr *h, uint64_t n,
                            const Fr *zinv)
 {
     const uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i < n) h[i] = (a[i] * b[i] - c[i]) * *zinv;
+    if (i < n) h[i] = (mul_any(a[i], b[i]) - c[i]) * *zinv;
 }
 
 // pass split: at most max_stages radix-2 stages per pass, spread evenly

@@ -13,7 +13,7 @@ template <class F>
 __device__ __forceinline__ F field_apply(int op, const F &a, const F &b)
 {
     switch (op) {
-    case 0: return a * b;
+    case 0: return mul_any(a, b);
     case 1: return a + b;
     case 2: return a - b;
     case 3: return sqr(a);
@@ -80,11 +80,11 @@ __global__ void k_group_op(int op, const F *a, const F *b, F *out, uint64_t n)
     const uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const F *pa = a + 3 * i;
-    const Affine<F> pa_aff = pa[2].is_zero() ? Affine<F>::inf() : Affine<F>{pa[0], pa[1]};
+    const Affine<F> pa_aff = pa[2].is_zero() ? Affine<F>::inf() : Affine<F>{reduced(pa[0]), reduced(pa[1])};
     Xyzz<F> r;
     if (op == 0) {
         const F *pb = b + 3 * i;
-        const Affine<F> pb_aff = pb[2].is_zero() ? Affine<F>::inf() : Affine<F>{pb[0], pb[1]};
+        const Affine<F> pb_aff = pb[2].is_zero() ? Affine<F>::inf() : Affine<F>{reduced(pb[0]), reduced(pb[1])};
         // exercise both the mixed and the XYZZ + XYZZ additions
         const Xyzz<F> xa = xyzz_add_affine(Xyzz<F>::inf(), pa_aff);
         const Xyzz<F> xb = xyzz_add_affine(Xyzz<F>::inf(), pb_aff);

@@ -34,7 +34,7 @@ __global__ void __launch_bounds__(256) k_spmv_products(SpmvArgs a, const Fr *__r
     const int m = blockIdx.y;
     const uint64_t k = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (k >= a.nu[m]) return;
-    a.prod[m][k] = a.nu_val[m][k] * z[a.nu_col[m][k]];
+    a.prod[m][k] = mul_any(a.nu_val[m][k], z[a.nu_col[m][k]]);
 }
 
 // phase 2: row sums of z[col] (unit terms) and prod[k] (the others)
