@@ -42,15 +42,16 @@ constexpr int kIcWin = 51, kIcDig = 16;       // signed 5-bit windows of a publi
 // need a third of the additions for the final sum, 32 are done sooner
 constexpr uint64_t kFewInputs = 64;
 
-// libff Jacobian (X, Y, Z) -> affine; Z = 0 is infinity
+// libff Jacobian (X, Y, Z) -> affine; Z = 0 is infinity.  Proofs come from anywhere: their
+// coordinates need not be reduced, the arithmetic after this wants them to be.
 template <class F>
 __device__ __forceinline__ Affine<F> libff_to_affine(const F *p)
 {
     if (p[2].is_zero()) return Affine<F>::inf();
-    if (p[2] == F::one()) return {p[0], p[1]};
+    if (p[2] == F::one()) return {reduced(p[0]), reduced(p[1])};
     const F zi = inverse(p[2]);
     const F zi2 = sqr(zi);
-    return {p[0] * zi2, p[1] * (zi2 * zi)};
+    return {zi2 * p[0], (zi2 * zi) * p[1]};
 }
 
 // gamma (lane 0) and delta (lane 1): Miller-loop lines; lanes also normalise ic

@@ -75,3 +75,33 @@ def test_products_and_spmv(ctx, times):
     want = ctx.spmv(n, n, ptr, col, vals, z)
     assert np.array_equal(ctx.spmv(n, n, ptr, col, _plus(vals, O.R, times), z), want)
     assert np.array_equal(ctx.spmv(n, n, ptr, col, vals, _plus(z, O.R, times)), want)
+
+
+@pytest.mark.parametrize("times", [1, 4, None])
+def test_pairing_and_verification(ctx, times):
+    rng = np.random.default_rng(64)
+    r1 = nk.generate("matmul", 2, 0, seed=9)
+    pk, vkp = nk.setup(ctx, r1, O.random_fr(5, rng))
+    be = nk.Backend(ctx)
+    be.prepare(r1, pk)
+    raw = be.prove(r1.witness)
+    r, s = O.random_fr(2, rng)
+    good = be.blind(raw, r, s)
+    proof = np.frombuffer(bytes(good), np.uint64).copy()
+    bad = proof.copy()
+    bad[36:48], bad[0:12] = proof[0:12], proof[36:48]
+    proofs = np.stack([proof, proof, proof, bad])
+    proofs[0, 0:8] = _plus(proofs[0, 0:8], O.P, times)      # A
+    proofs[1, 36:44] = _plus(proofs[1, 36:44], O.P, times)  # C
+    proofs[2, 12:28] = _plus(proofs[2, 12:28], O.P, times)  # B
+    proofs[3, 0:8] = _plus(proofs[3, 0:8], O.P, times)
+    pub = np.ascontiguousarray(r1.witness[1:1 + r1.public_inputs])
+    publics = np.stack([pub, pub, _plus(pub, O.R, times), pub])
+    vk = nk.VerifyingKey(ctx, vkp["alpha_g1_beta_g2"], vkp["gamma_g2"], vkp["delta_g2"], vkp["ic"])
+    assert vk.verify_batch(publics, proofs).tolist() == [True, True, True, False]
+    vk.free()
+    p, q = proof[0:12].copy(), proof[12:36].copy()
+    want = nk.reduced_pairing(ctx, p[None], q[None])
+    p[:8], q[:16] = _plus(p[:8], O.P, times), _plus(q[:16], O.P, times)
+    assert np.array_equal(nk.reduced_pairing(ctx, p[None], q[None]), want)
+    be.free()
