@@ -469,12 +469,28 @@ __global__ void __launch_bounds__(32) k_blind_proof(const BlindSums *sums, const
 
 bool is_one(const host::Fq &z) { return z == host::Fq::one(); }
 
+// The values below p of n coordinates (a raw proof comes from the caller; the kernels take
+// coordinates below 2p)
+void reduce_coordinates(uint8_t *p, int n)
+{
+    for (int i = 0; i < n; ++i) {
+        host::Fq x;
+        std::memcpy(x.v, p + 32 * i, 32);
+        if (!host::geq_mod<host::FqMod>(x.v)) continue;
+        x = x * host::Fq::one();
+        std::memcpy(p + 32 * i, x.v, 32);
+    }
+}
+
 // Affine-normalise a libff point held as Z = 1, Z = 0 (infinity) or anything else.
 void normalize_g1_if_needed(uint8_t *p)
 {
     host::Fq z;
     std::memcpy(z.v, p + 64, 32);
-    if (!z.is_zero() && !is_one(z)) host::normalize_g1(p);
+    if (!z.is_zero() && !is_one(z))
+        host::normalize_g1(p);
+    else
+        reduce_coordinates(p, 2);
 }
 
 void normalize_g2_if_needed(uint8_t *p)
@@ -483,7 +499,10 @@ void normalize_g2_if_needed(uint8_t *p)
     std::memcpy(z0.v, p + 128, 32);
     std::memcpy(z1.v, p + 160, 32);
     const bool inf = z0.is_zero() && z1.is_zero();
-    if (!inf && !(is_one(z0) && z1.is_zero())) host::normalize_g2(p);
+    if (!inf && !(is_one(z0) && z1.is_zero()))
+        host::normalize_g2(p);
+    else
+        reduce_coordinates(p, 4);
 }
 
 } // namespace

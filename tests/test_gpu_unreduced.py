@@ -105,3 +105,22 @@ def test_pairing_and_verification(ctx, times):
     p[:8], q[:16] = _plus(p[:8], O.P, times), _plus(q[:16], O.P, times)
     assert np.array_equal(nk.reduced_pairing(ctx, p[None], q[None]), want)
     be.free()
+
+
+@pytest.mark.parametrize("times", [1, 4, None])
+def test_blinding(ctx, times):
+    rng = np.random.default_rng(65)
+    r1 = nk.generate("matmul", 2, 0, seed=9)
+    pk, _ = nk.setup(ctx, r1, O.random_fr(5, rng))
+    be = nk.Backend(ctx)
+    be.prepare(r1, pk)
+    raw = be.prove(r1.witness)
+    r, s = O.random_fr(2, rng)
+    want = bytes(be.blind(raw, r, s))
+    again = type(raw).from_buffer_copy(bytes(raw))
+    words = np.frombuffer(again, np.uint64)
+    for i in range(4):
+        words[12 * i:12 * i + 8] = _plus(words[12 * i:12 * i + 8], O.P, times)
+    words[48:64] = _plus(words[48:64], O.P, times)
+    assert bytes(be.blind(again, r, s)) == want
+    be.free()
