@@ -507,22 +507,33 @@ int key_prove(nkr_b200_key *key, const void *witness, uint64_t n, nkr_b200_raw_p
     cudaStream_t s0 = sl->main();
     // s0 is ordered after the previous prove's joins, so z is free to overwrite
     NKR_CUDA(cudaMemcpyAsync(sl->z.p, witness, n * 32, copy_kind_from(witness), s0));
-    // The first prove of a key issues its launches, the second captures them as well: a
-    // prove is some 150 launches on 17 streams, about 0.7 ms of host work, and a program
-    // that proves once does not pay for the capture.  Replayed, a prove and blinding of a
-    // 16-step circuit takes 0.71 ms (issued 0.77), of matmul 32 1.49 ms (1.53), of 2^20
-    // constraints 10.03 ms (10.17).
-    if (sl->proves == 0) {
-        NKR_TRY(prove_issue(key, sl, true, true));
-    } else {
-        if (!sl->single.exec) {
-            sl->single.release();
-            NKR_TRY(capture_prove(key, sl, true, true, true, &sl->single));
-        }
-        NKR_CUDA(cudaGraphLaunch(sl->single.exec, s0));
-        g_kernel_launches.fetch_add(sl->single.kernels, std::memory_order_relaxed);
-    }
-    ++sl->proves;
+    // The first prove of a key issues its launches, the second captures them and those after
+    // it replay: a prove is some 150 launches on 17 streams, about 0.7 ms of host work.
+    // Replayed, a prove and blinding of a 16-step circuit takes 0.71 ms (issued 0.77), of
+    // matmul 32 1.49 ms (1.53), of 2^20 constraints 10.03 ms (10.17).  The capture makes the
+    // second prove longer by 1.3 ms (16 steps: 1.90 ms, then 0.62), 0.7 ms (matmul 32: 2.02,
+    // then 1.34) and 1.4 ms (2^20: 10.5, then 9.1).
+    NKR_TRY(sl->replay.run([&] { return sl->single.exec != nullptr; },
+                           [&] {
+                               const int s = capture_prove(key, sl, true, true, true, &sl->single);
+                               if (s != NKR_B200_OK) {
+                                   cudaGetLastError(); // not the issued launches' error
+                                   sl->single.release();
+                               }
+                               return s;
+                           },
+                           [&] {
+                               const cudaError_t e = cudaGraphLaunch(sl->single.exec, s0);
+                               if (e != cudaSuccess) {
+                                   cudaGetLastError();
+                                   sl->single.release();
+                                   set_error("prove graph launch failed: %s", cudaGetErrorString(e));
+                                   return int(NKR_B200_ECUDA);
+                               }
+                               g_kernel_launches.fetch_add(sl->single.kernels, std::memory_order_relaxed);
+                               return int(NKR_B200_OK);
+                           },
+                           [&] { return prove_issue(key, sl, true, true); }));
     NKR_CUDA(cudaMemcpyAsync(sl->pinned_out, sl->out.p, kOutBytes, cudaMemcpyDeviceToHost, s0));
     NKR_CUDA(cudaStreamSynchronize(s0));
     normalize_raw(sl->pinned_out);

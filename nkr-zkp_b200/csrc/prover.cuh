@@ -26,6 +26,7 @@
 #include "field.cuh"
 #include "msm.cuh"
 #include "ntt.cuh"
+#include "replay.hpp"
 #include "spmv.cuh"
 
 struct nkr_b200_ctx {
@@ -94,7 +95,7 @@ struct ProveSlot {
     // the stream it is launched into; and of nkr_b200_prove (slot 0: stage events, blinding
     // tables), whose kernels keep their streams' priorities
     ProveGraph batch, single;
-    uint64_t proves = 0; // nkr_b200_prove calls on this slot
+    ReplayPolicy replay; // of nkr_b200_prove
     // pinned staging: witness double buffer (pageable inputs) and results
     void *pinned_wit[2] = {nullptr, nullptr};
     cudaEvent_t ev_wit[2] = {nullptr, nullptr};
