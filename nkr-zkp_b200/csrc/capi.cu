@@ -444,10 +444,7 @@ int nkr_b200_msm_bases_create(nkr_b200_ctx *ctx, int group, const void *bases, u
     h->ctx = ctx;
     std::vector<uint32_t> idx = msm_support(group, bases, n);
     int c = 0;
-    // the widths are measured on G1; a G2 addition of the reduction levels takes some four
-    // times as long, a G2 entry of level 1 three times, so G2 takes the width of a quarter of
-    // the points (100,001 points: 15 bits 1.65 ms, 16 bits 1.72 ms, 17 bits 1.81 ms)
-    NKR_TRY(tuned_window_bits(ctx, group == 1 ? idx.size() : (idx.size() + 3) / 4, &c));
+    NKR_TRY(tuned_window_bits(ctx, group == 1 ? idx.size() : g2_width_size(idx.size()), &c));
     NKR_TRY(msm_bases_build_support(h->bases, group, bases, n, std::move(idx), true, c, ctx->stream));
     NKR_TRY(msm_scratch_alloc(h->scratch, group, h->bases.shape));
     for (auto &e : h->scratch.acc.ev_acc) NKR_CUDA(cudaEventCreate(&e));

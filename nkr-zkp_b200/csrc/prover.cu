@@ -434,7 +434,9 @@ int key_prepare(nkr_b200_ctx *ctx, const nkr_b200_circuit *c, const nkr_b200_pro
     NKR_PREP(ntt_tables_build(key->ntt, logn, st));
     // proving key: normalise (hazard: CPU-setup keys are unnormalised Jacobian), fold
     // windows; witness queries keep only their finite points (variables present in the matrix)
-    // window widths from the autotuner (per support size; 0 = cost model)
+    // window widths from the autotuner (per support size; 0 = cost model).  The B query on G2
+    // keeps G1's width: its digit sort is then the one of the B query on G1, and its
+    // reduction levels run beside other MSMs' level 1.
     const void *wq[4] = {pk->a_query, pk->b_g1_query, pk->l_query, pk->b_g2_query};
     const int wk[4] = {kMsmA, kMsmB1, kMsmL, kMsmB2};
     for (int j = 0; j < 4; ++j) {

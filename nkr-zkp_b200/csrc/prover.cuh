@@ -45,6 +45,8 @@ namespace nkr {
 // on this device when autotuning is on (synthetic bases, uniform scalars),
 // else 0 (the cost model).  Sizes above 2^22 take the 2^22 offset from the model.
 int tuned_window_bits(nkr_b200_ctx *ctx, uint64_t n, int *c);
+// the number of points whose width resident G2 bases of n points take
+uint64_t g2_width_size(uint64_t n);
 } // namespace nkr
 
 namespace nkr {

@@ -7,6 +7,7 @@
 // the model's c and its neighbours, once per power-of-two size class, and keeps
 // the fastest.  Any c gives the same (canonical) result.
 #define NKR_FIELD_MUL_OUTLINE 1
+#include <algorithm>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -148,6 +149,26 @@ int measure(nkr_b200_ctx *ctx, int lg)
 }
 
 } // namespace
+
+// The widths are measured on G1.  A bucket of a G2 MSM costs the reduction levels more,
+// against an entry of level 1, so G2 takes the width of fewer points:
+//   up to 2^12 the smallest size that is tuned (the whole MSM is latency: every bit of the
+//     width is another step of the reduction), up to 2^15 half of the points, up to 2^19 a
+//     quarter, and beyond all of them (level 1 dominates and a narrower width adds entries).
+// Measured on G2, ms with uniform / sparse scalars for the widths of all, half and a quarter
+// of the points (below 2^12: all, the smallest, a quarter or else the model's):
+//     1,500  0.47 / 0.50  0.42 / 0.45  0.46 / 0.48      3,001  0.57 / 0.52  0.48 / 0.38  0.48 / 0.38
+//     8,192  0.61 / 0.57  0.61 / 0.55  0.64 / 0.61     12,000  0.68 / 0.58  0.68 / 0.58  0.80 / 0.58
+//    50,000  1.28 / 0.81  1.27 / 0.81  1.25 / 0.75    100,001  1.73 / 0.97  1.68 / 0.90  1.69 / 0.91
+//   200,000  2.74 / 1.18  2.73 / 1.18  2.72 / 1.23    262,144  3.31 / 1.46  3.32 / 1.46  3.37 / 1.37
+//      2^20  9.70 / 2.43  11.4 / 2.60  11.4 / 2.60 (17 and 16 bits)
+uint64_t g2_width_size(uint64_t n)
+{
+    if (n <= uint64_t(1) << 12) return std::min(n, uint64_t(1) << kTuneMinLog);
+    if (n <= uint64_t(1) << 15) return (n + 1) / 2;
+    if (n <= uint64_t(1) << 19) return (n + 3) / 4;
+    return n;
+}
 
 int tuned_window_bits(nkr_b200_ctx *ctx, uint64_t n, int *c)
 {
