@@ -315,7 +315,9 @@ int nkr_b200_msm_g2(nkr_b200_ctx *ctx, const void *bases, const void *scalars, u
 /* MSM window autotuner (on by default; environment NKR_B200_AUTOTUNE=0 turns it
  * off).  The window width of every resident MSM (prepare, msm_bases_create) is
  * measured once per power-of-two size class on this device: the cost model's
- * width and its neighbours are timed on synthetic bases and the fastest kept.
+ * width and its neighbours are timed on synthetic G1 bases and the fastest kept, or
+ * one within 3% of it that does less work.  Resident G2 bases take the width of
+ * fewer points (tune.cu).
  * nkr_b200_tune_msm returns (and, if needed, measures) the width for n points and
  * the measured MSM time at that size class (0 when the size is not measured).
  * Replaces choose_window_bits (backends/cuda/src/groth16_backend.cu:17-25: 8, 11

@@ -5,7 +5,7 @@
 // bound, so its real cost per bucket depends on the part and the size.  The
 // tuner times the whole MSM (sort + accumulation + reduction) on this device for
 // the model's c and its neighbours, once per power-of-two size class, and keeps
-// the fastest.  Any c gives the same (canonical) result.
+// the fastest, or one within 3% of it that does less work (width_choice.hpp).  Any c gives the same (canonical) result.
 #define NKR_FIELD_MUL_OUTLINE 1
 #include <algorithm>
 #include <cstdio>
@@ -16,6 +16,7 @@
 
 #include "msm.cuh"
 #include "prover.cuh"
+#include "width_choice.hpp"
 
 namespace nkr {
 
@@ -101,8 +102,6 @@ int measure(nkr_b200_ctx *ctx, int lg)
     NKR_CUDA(cudaEventCreate(&e0));
     NKR_CUDA(cudaEventCreate(&e1));
     const int c0 = msm_shape(n, true, 1).c;
-    int best_c = c0;
-    float best = 1e30f;
     std::vector<std::pair<int, float>> times;
     int status = NKR_B200_OK;
     for (int c = c0 - 3; c <= c0 + 1 && status == NKR_B200_OK; ++c) {
@@ -127,24 +126,13 @@ int measure(nkr_b200_ctx *ctx, int lg)
             if (rep > 0 && ms < t_min) t_min = ms; // rep 0 warms up
         }
         times.push_back({c, t_min});
-        if (t_min < best) best = t_min;
-    }
-    // Widths within 3% of the fastest alone differ in the work that they leave for others:
-    // of these the one of the least work is kept (a batch of 8 proofs of 2^15 constraints
-    // took 7.0 to 7.7 ms with whichever happened to be the fastest)
-    double least = 1e300;
-    for (const auto &[c, t] : times) {
-        const double work = msm_work(n, c);
-        if (t <= 1.03f * best && work < least) {
-            least = work;
-            best_c = c;
-        }
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     if (status != NKR_B200_OK) return status;
-    ctx->msm_window[lg] = best_c;
-    ctx->msm_window_ms[lg] = best;
+    const auto choice = choose_width(times, [&](int c) { return msm_work(n, c); });
+    ctx->msm_window[lg] = choice.first;
+    ctx->msm_window_ms[lg] = choice.second;
     return NKR_B200_OK;
 }
 
