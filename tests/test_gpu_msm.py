@@ -234,3 +234,63 @@ def test_msm_full_size_equals_scalar_sum(ctx, orc, rng, group, logn, mix):
     got, _ = b.run(sc)
     b.free()
     assert np.array_equal(got, want)
+
+
+@pytest.mark.parametrize("group", [1, 2])
+def test_large_buckets_where_16_pieces_are_summed_with_the_bucket(orc, rng, group):
+    """600,000 points with 17-bit windows: buckets of up to 16 level-1 pieces are summed by
+    the first reduction level, larger ones by the fix-up levels.  Buckets of 15 to 65 whole
+    segments, and of one entry less and more, so that the ones behind them are ragged."""
+    n = 600_000
+    ctx = nk.Context(0)
+    ctx.set_autotune(False)
+    ks = O.random_fr(37, rng)
+    gen = orc.g1_generator() if group == 1 else orc.g2_generator()
+    pts = np.stack([orc.mul_affine(group, gen, k) for k in ks])
+    at = np.arange(n) % 37
+    b = nk.MsmBases(ctx, group, O.affine_to_jac(group, pts)[at])
+    tab = np.stack([O.fr_mont(v) for v in range(1 << 16)])
+    kint = [O.fr_int(k) for k in ks]
+
+    def run(values):
+        got, _ = b.run(tab[values])
+        per = [int(values[at == j].sum()) for j in range(37)]
+        total = sum(p * k for p, k in zip(per, kint)) % O.R
+        want = O.affine_to_jac(group, orc.mul_affine(group, gen, O.fr_mont(total)))[0]
+        assert np.array_equal(got, want)
+        return b.stats()
+
+    st = run(rng.integers(1, 1 << 16, n))
+    # buckets of up to 16 pieces (not 4) where entries may fill all buckets with 4 segments of 32
+    assert st["window_bits"] == 17 and n * st["windows"] >= 4 * 32 * st["buckets"] and st["entries"] == n
+    seg = -(-n // st["tasks"])
+    assert -(-n // seg) == st["tasks"] and seg > 4
+    pieces = (15, 16, 17, 64, 65)
+    sizes = [p * seg for p in pieces] + [p * seg + d for p in pieces for d in (-1, 1)] + [1, seg, 4 * seg, 5 * seg]
+    for front in (0, 1): # aligned with the segments, and one entry off
+        values = rng.integers(100, 1 << 16, n)
+        head = np.repeat(np.arange(1, 2 + len(sizes)), [front] + sizes)
+        values[:head.size] = head
+        assert run(rng.permutation(values))["entries"] == n
+    b.free()
+    ctx.close()
+
+
+@pytest.mark.parametrize("group", [1, 2])
+def test_statistics_of_runs(ctx, orc, rng, group):
+    """Zero before a run; then the last run's phases, read when they are asked for, and its
+    entries: one per nonzero digit."""
+    n = 3000
+    b = nk.MsmBases(ctx, group, O.affine_to_jac(group, _points(orc, group, n, rng, distinct=5)))
+    assert not any(b.stats().values())
+    phases = ("sort_ms", "acc_ms", "fixup_ms", "reduce_first_ms", "reduce_levels_ms")
+    for value, entries in ((1, n), (0, 0), (1, n)):
+        sc = np.tile(O.fr_mont(value), (n, 1))
+        sc[7] = 0
+        _, ms = b.run(sc)
+        st = b.stats()
+        assert st == b.stats() and abs(st["total_ms"] - ms) < 1e-6
+        assert st["entries"] == max(entries - 1, 0) and (st["tasks"] > 0) == (entries > 0)
+        assert all(st[p] >= 0 for p in phases) and st["acc_ms"] > 0
+        assert sum(st[p] for p in phases) <= st["total_ms"] + 5e-3  # 1 us of resolution a phase
+    b.free()

@@ -174,14 +174,16 @@ def test_prepare_rejects_bad_shapes(ctx):
 
 
 def test_prove_repeated_witness_values(ctx, ref, tmp_path):
-    """Repeated witness values go through the class path of the G1 witness MSMs:
-    variables of equal value form a class whose bases are summed once, and a small
-    MSM over the class values adds v_c S_c.  A crafted witness with more
+    """Repeated witness values go through the class path of the witness MSMs (circuits
+    of more than 2^16 variables): variables of equal value form a class whose bases
+    are summed once, and a small MSM over the class values adds v_c S_c.  A crafted
+    witness with more
     minimum-size classes (4 members) than one prove takes (4,096; the others stay
     singletons), groups below the minimum, large classes (fix-up levels), values
     beside their negations and zeros gives the reference CPU prover's raw proof,
     before and after a prove of the circuit's own witness on the same slot."""
-    r1 = nk.generate("matmul", 32, 0, seed=31)
+    r1 = nk.generate("matmul", 40, 0, seed=31)
+    assert r1.cols > 1 << 16
     pk_path, vk_path = tmp_path / "c.pk.bin", tmp_path / "c.vk.bin"
     ref.cpu_setup(r1, pk_path, vk_path)
     pk = O.read_proving_key(pk_path)
