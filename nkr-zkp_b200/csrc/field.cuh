@@ -16,14 +16,6 @@
 
 namespace nkr {
 
-// True for a field type whose products have a paired form mul2 (two independent
-// products in one call; field52.cuh).  The curve formulas issue their products in
-// pairs only for such fields and keep their original order otherwise.
-template <class F>
-struct HasPairedMul {
-    static constexpr bool value = false;
-};
-
 struct FqParams {
     static constexpr uint32_t P0 = 0xd87cfd47u, P1 = 0x3c208c16u, P2 = 0x6871ca8du,
                               P3 = 0x97816a91u, P4 = 0x8181585du, P5 = 0xb85045b6u,

@@ -266,16 +266,6 @@ __device__ __forceinline__ void mul52x2(const Fq52 &a, const Fq52 &b, const Fq52
 
 __device__ __forceinline__ Fq52 operator*(const Fq52 &a, const Fq52 &b) { return mul52(a, b); }
 __device__ __forceinline__ Fq52 sqr(const Fq52 &a) { return mul52(a, a); }
-// x = a b, y = c d (curve formulas issue independent products in pairs)
-__device__ __forceinline__ void mul2(const Fq52 &a, const Fq52 &b, const Fq52 &c, const Fq52 &d,
-                                     Fq52 &x, Fq52 &y)
-{
-    mul52x2(a, b, c, d, x, y);
-}
-template <>
-struct HasPairedMul<Fq52> {
-    static constexpr bool value = true;
-};
 
 __device__ __forceinline__ Fq52 operator+(const Fq52 &a, const Fq52 &b)
 {
@@ -363,34 +353,8 @@ __device__ NKR_MUL52_ATTR Fq52L mul52L(Fq52L a, Fq52L b)
     return r;
 }
 
-struct Fq52LPair {
-    Fq52L x, y;
-};
-
-// (a b, c d) in one call, lazily reduced (as mul52x2v)
-__device__ NKR_MUL52_ATTR Fq52LPair mul52Lx2v(Fq52L a, Fq52L b, Fq52L c, Fq52L d)
-{
-    Fq52LPair r;
-    const Fq52L *pa[2] = {&a, &c}, *pb[2] = {&b, &d};
-    Fq52L *pr[2] = {&r.x, &r.y};
-    mul52_body<2>(pa, pb, pr);
-    return r;
-}
-
 __device__ __forceinline__ Fq52L operator*(const Fq52L &a, const Fq52L &b) { return mul52L(a, b); }
 __device__ __forceinline__ Fq52L sqr(const Fq52L &a) { return mul52L(a, a); }
-
-__device__ __forceinline__ void mul2(const Fq52L &a, const Fq52L &b, const Fq52L &c, const Fq52L &d,
-                                     Fq52L &x, Fq52L &y)
-{
-    const Fq52LPair r = mul52Lx2v(a, b, c, d);
-    x = r.x;
-    y = r.y;
-}
-template <>
-struct HasPairedMul<Fq52L> {
-    static constexpr bool value = true;
-};
 
 // (a + b) mod 2p for a, b in [0, 2p)
 __device__ __forceinline__ Fq52L operator+(const Fq52L &a, const Fq52L &b)
@@ -469,26 +433,6 @@ __device__ __forceinline__ Fq2x52 sqr(const Fq2x52 &a)
     Fq52 p, q;
     mul52x2(a.c0 + a.c1, a.c0 - a.c1, a.c0, a.c1, p, q);
     return {p, q + q};
-}
-
-// Fermat inverse a^(p-2); R' products keep the R' domain.  0 maps to 0.
-__device__ inline Fq52 inverse(const Fq52 &a)
-{
-    const uint32_t e[8] = {FqParams::P0 - 2u, FqParams::P1, FqParams::P2, FqParams::P3,
-                           FqParams::P4,      FqParams::P5, FqParams::P6, FqParams::P7};
-    Fq52 acc = Fq52::one();
-    for (int i = 255; i >= 0; --i) {
-        acc = sqr(acc);
-        if ((e[i >> 5] >> (i & 31)) & 1) acc = acc * a;
-    }
-    return acc;
-}
-
-// 1 / (a0 + a1 u) = (a0 - a1 u) / (a0^2 + a1^2)
-__device__ inline Fq2x52 inverse(const Fq2x52 &a)
-{
-    const Fq52 ni = inverse(sqr(a.c0) + sqr(a.c1));
-    return {a.c0 * ni, neg(a.c1) * ni};
 }
 
 // ---------------------------------------------------------------------------

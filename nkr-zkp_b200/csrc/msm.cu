@@ -1657,11 +1657,4 @@ int msm_result_add(int group, void *out_dev, const void *add_dev, cudaStream_t s
     return NKR_B200_OK;
 }
 
-int msm_class_acc_run(const MsmBases &b, const MsmClassSort &cs, const MsmDedup &d, MsmClassAcc &a,
-                      void *out_dev, cudaStream_t st)
-{
-    NKR_TRY(msm_class_acc_issue(b, cs, d, a, st));
-    return msm_result_add(b.group, out_dev, a.out.p, st);
-}
-
 } // namespace nkr

@@ -273,12 +273,8 @@ struct MsmClassAcc {
     }
 };
 int msm_class_acc_alloc(MsmClassAcc &a, int group, uint64_t n);
-// Class sums over bases b (its first n points: 2^0 window copies), the MSM over
-// the classes, and out_dev (the MSM's result, libff Jacobian) += that sum.
-int msm_class_acc_run(const MsmBases &b, const MsmClassSort &cs, const MsmDedup &d, MsmClassAcc &a,
-                      void *out_dev, cudaStream_t st);
-// the class-path part of msm_class_acc_run without the final addition (a.out
-// holds sum_c v_c S_c), and the addition alone
+// Class sums over bases b (its first n points: 2^0 window copies) and the MSM over the
+// classes: a.out = sum_c v_c S_c; and out_dev (the MSM's result, libff Jacobian) += add_dev.
 int msm_class_acc_issue(const MsmBases &b, const MsmClassSort &cs, const MsmDedup &d, MsmClassAcc &a,
                         cudaStream_t st);
 int msm_result_add(int group, void *out_dev, const void *add_dev, cudaStream_t st);

@@ -1,16 +1,16 @@
 // Points held by four lanes.  Lane role r = lane & 3 keeps coordinate r of an XYZZ
 // point (0: X, 1: Y, 2: ZZ, 3: ZZZ) and the four lanes compute one product each at a
-// time: an addition's 14 products take 4 steps, a mixed addition's 10 take 4, a
-// doubling's 9 take 3, with the operands exchanged by shuffles between the steps.
+// time: an addition's 14 products take 4 steps, a doubling's 9 take 3, with the operands
+// exchanged by shuffles between the steps.
 //
 // This is for chains of dependent additions run by few threads (bucket reduction,
-// fix-ups, Horner passes, level 1 of small MSMs), where a field product is pure latency
+// fix-ups, Horner passes, blinding), where a field product is pure latency
 // (about 440 ns for a warp alone on its scheduler): one addition by one thread took
 // 5 to 8 us there, by four lanes about 2 us.  A lane keeps one coordinate of each
 // point, so the G2 forms need no local memory either (one thread holding whole G2
 // points spilled up to 2.5 KB).
 //
-// The formulas are those of curve.cuh (add-2008-s, madd-2008-s, dbl-2008-s-1) with the
+// The formulas are those of curve.cuh (add-2008-s, dbl-2008-s-1) with the
 // same treatment of infinity (ZZ = 0), equal and opposite points.  All four lanes of a
 // quad take every branch together; other quads of the warp may be elsewhere.
 #pragma once
@@ -87,23 +87,6 @@ __device__ __forceinline__ C quad_dbl(const C &v)
     return role == 0 ? x3 : role == 1 ? y3 : role == 2 ? g : h;
 }
 
-// The steps after the first products: lanes 0 and 1 hold U1 and S1 in m and
-// P and R in d, lane 2 and 3 the product of the ZZ and of the ZZZ in z.
-template <class C>
-__device__ __forceinline__ C quad_add_tail(const C &m, const C &d, const C &z, const C &s)
-{
-    const unsigned role = quad_role();
-    // lane 0: Q = U1 PP, 1 and 3: PPP = P PP, 2: ZZ' = ZZ12 PP
-    const C pp = quad_get(s, 0), p = quad_get(d, 0);
-    const C g = (role == 0 ? m : role == 2 ? z : p) * pp;
-    const C rr = quad_get(s, 1), ppp = quad_get(g, 1), r = quad_get(d, 1);
-    const C x3 = rr - ppp - dbl(g);          // lane 0
-    // lane 0: R (Q - X'), 1: S1 PPP, 3: ZZZ' = ZZZ12 PPP
-    const C h = (role == 0 ? r : role == 1 ? m : z) * select(role == 0, g - x3, g);
-    const C y3 = quad_get(h, 0) - h;         // lane 1
-    return role == 0 ? x3 : role == 1 ? y3 : role == 2 ? g : h;
-}
-
 // a + b
 template <class C>
 __device__ __forceinline__ C quad_add(const C &a, const C &b)
@@ -121,24 +104,15 @@ __device__ __forceinline__ C quad_add(const C &a, const C &b)
     if (quad_flag(z, 0)) return quad_flag(z, 1) ? quad_dbl(a) : quad_inf<C>();
     // lane 0: PP, 1: RR, 2: ZZ1 ZZ2, 3: ZZZ1 ZZZ2
     const C s = select(low, d, a) * select(low, d, b);
-    return quad_add_tail(m, d, s, s);
-}
-
-// a + q for an affine point q that is not infinity, q = x in lanes 0, 2 and y in
-// lanes 1, 3
-template <class C>
-__device__ __forceinline__ C quad_add_affine(const C &a, const C &q)
-{
-    const unsigned role = quad_role();
-    if (quad_is_inf(a)) return role < 2 ? q : C::one();
-    const bool low = role < 2;
-    const C m = select(low, a, a * q);       // lane 2: U2 = X2 ZZ1, 3: S2 = Y2 ZZZ1
-    const C n = quad_get(m, int(role ^ 2u));
-    const C d = select(low, n, m) - select(low, m, n);
-    const bool z = d.is_zero();
-    if (quad_flag(z, 0)) return quad_flag(z, 1) ? quad_dbl(a) : quad_inf<C>();
-    const C s = d * d;                       // lane 0: PP, 1: RR
-    return quad_add_tail(a, d, a, s);
+    // lane 0: Q = U1 PP, 1 and 3: PPP = P PP, 2: ZZ' = ZZ12 PP
+    const C pp = quad_get(s, 0), p = quad_get(d, 0);
+    const C g = (role == 0 ? m : role == 2 ? s : p) * pp;
+    const C rr = quad_get(s, 1), ppp = quad_get(g, 1), r = quad_get(d, 1);
+    const C x3 = rr - ppp - dbl(g);          // lane 0
+    // lane 0: R (Q - X'), 1: S1 PPP, 3: ZZZ' = ZZZ12 PPP
+    const C h = (role == 0 ? r : role == 1 ? m : s) * select(role == 0, g - x3, g);
+    const C y3 = quad_get(h, 0) - h;         // lane 1
+    return role == 0 ? x3 : role == 1 ? y3 : role == 2 ? g : h;
 }
 
 } // namespace nkr
