@@ -172,7 +172,7 @@ int nkr_b200_vk_prepare(nkr_b200_ctx *ctx, const nkr_b200_verification_key *vk,
                         nkr_b200_vk **out);
 
 /* Replaces verify (common/src/protocol.cpp:96-108) for a batch of count proofs
- * of one key, one proof per GPU thread.  proofs: count nkr_b200_proof records
+ * of one key, six lanes per proof.  proofs: count nkr_b200_proof records
  * (A, B, C in libff layout, any Z) in host memory; public_inputs: count rows of
  * n_public Fr (Montgomery, 32 B each).  accept[i] = 1 when proof i satisfies
  * e(A, B) = e(alpha, beta) e(vk_x, gamma) e(C, delta), else 0; as in the
@@ -367,8 +367,8 @@ uint64_t nkr_b200_launch_count(void);
 
 /* Elementwise field op over n pairs (host buffers): field 0 Fr, 1 Fq, 2 Fq2;
  * op 0 mul, 1 add, 2 sub, 3 sqr, 4 inverse, 5 to_mont, 6 from_mont.  Fields 3
- * (Fq) and 4 (Fq2) run ops 0..3 and 4 = negation in the MSM's FP64-limb
- * arithmetic (same inputs and outputs as fields 1 and 2). */
+ * (Fq) and 4 (Fq2) run ops 0..3 and 4 = negation in FP64-limb arithmetic (same
+ * inputs and outputs as fields 1 and 2). */
 int nkr_b200_field_op(nkr_b200_ctx *ctx, int field, int op, const void *a, const void *b,
                       void *out, uint64_t n);
 /* Elementwise group op: group 1 G1, 2 G2; inputs affine-normalised Jacobian layout.

@@ -1,8 +1,9 @@
 // BN254 base field Fq and scalar field Fr on sm_100a.
 //
 // Representation: 8 x 32-bit little-endian limbs in Montgomery form
-// (R = 2^256), always fully reduced (< modulus).  The byte image is identical
-// to libff's Fp_model<4, modulus>::mont_repr on x86-64, so device buffers are
+// (R = 2^256), in memory always fully reduced (< modulus); kernels compute in Fp, fully
+// reduced as well, or on values below twice the modulus (FpL, Fq2M).  The byte image is
+// identical to libff's Fp_model<4, modulus>::mont_repr on x86-64, so device buffers are
 // bit-for-bit the reference's host vectors (reference: libff
 // algebra/fields/fp.hpp:40-42, CUDA mont_t layout operators/cuda/include/fields/
 // mont_t.cuh:45).
@@ -925,12 +926,10 @@ __device__ __forceinline__ uint32_t p2_word(int k)
 } // namespace lazy
 
 // Fq2 with the lazily reduced product below: same layout and values as Fq2, its
-// arithmetic closed over the type.  It is the compute type of the G2 bucket
-// reduction levels, whose long dependent chains gain from the shorter product
-// (at 2^18 points: first level 0.41 -> 0.36 ms, block levels 1.50 -> 1.22 ms);
-// the G2 accumulation keeps Fq2, where the larger product body costs registers:
-// 255 with spills at 2 blocks per SM (4% slower), 100 B of spills at the 3-block
-// budget of the shared-memory accumulator (3.86 instead of 3.25 ms at 2^18).
+// arithmetic closed over the type.  It is the compute type of lane quads on G2 (the MSM's
+// levels after the first, blinding), whose long dependent chains gain from the shorter
+// product; the G2 accumulation takes Fq2M, where this product's live values spill
+// (100,001 points 1.94 ms, with Fq2M 1.84).
 struct Fq2L : Fq2 {
     Fq2L() = default;
     __device__ __forceinline__ Fq2L(const Fq2 &a) : Fq2(a) {}

@@ -1,8 +1,9 @@
 // Fq in five 52-bit limbs with products on the double-precision FMA pipe.
 //
-// The Montgomery product of field.cuh is bound by the integer multiply (IMAD)
-// pipe and, for one warp alone, by its long carry chains (about a microsecond
-// of latency per product).  B200 also has a full-rate FP64 pipe, and a double
+// The alternative to the integer product of field.cuh, which is as fast (63.7e9 products/s
+// in registers against 63.5 to 65.2e9 here) with fewer registers and conversions, so that
+// the kernels use that one; this is here for the field operations and microbenchmarks of the
+// C interface that compare the two.  B200 has a full-rate FP64 pipe, and a double
 // FMA computes a 52 x 52-bit limb product exactly when the high half is taken
 // with round toward zero against a 2^104 offset and the low half as the exact
 // remainder (Emmart, Zheng and Weems, "Faster modular exponentiation using
@@ -18,8 +19,7 @@
 //
 // Representation: limbs are uint64 integers < 2^52, values canonical (< p),
 // Montgomery form with R' = 2^260.  In memory these values are stored in the
-// 8 x 32-bit layout of Fq (to52 / from52 only move bits); the MSM keeps all of
-// its buffers in the R' domain and converts at entry (bases) and exit (result).
+// 8 x 32-bit layout of Fq (to52 / from52 only move bits).
 #pragma once
 
 #include <cstdint>
@@ -312,8 +312,7 @@ __device__ __forceinline__ Fq52 dbl(const Fq52 &a) { return a + a; }
 // 1.05 p (mul52_body), so it skips the conditional subtraction of p that ends a
 // canonical product (about 40 of its 362 instructions); additions and
 // subtractions work modulo 2p at the cost of their canonical forms.  Zero tests
-// accept 0 and p.  MSM kernels compute in this type and canonicalise once, when a
-// value leaves for memory (canon()).
+// accept 0 and p.
 // ---------------------------------------------------------------------------
 struct Fq52L {
     uint64_t l[5];
@@ -420,9 +419,7 @@ __device__ __forceinline__ Fq2x52 operator-(const Fq2x52 &a, const Fq2x52 &b)
 }
 __device__ __forceinline__ Fq2x52 neg(const Fq2x52 &a) { return {neg(a.c0), neg(a.c1)}; }
 __device__ __forceinline__ Fq2x52 dbl(const Fq2x52 &a) { return {dbl(a.c0), dbl(a.c1)}; }
-// Karatsuba, the three base-field products in one call (the FP64 Fq2 form serves
-// latency-bound single-thread chains, where one call of three interleaved
-// products takes far less than a pair and a single)
+// Karatsuba, the three base-field products in one call, their chains interleaved
 __device__ __forceinline__ Fq2x52 operator*(const Fq2x52 &a, const Fq2x52 &b)
 {
     const Fq52Triple t = mul52x3v(a.c0, b.c0, a.c1, b.c1, a.c0 + a.c1, b.c0 + b.c1);

@@ -141,8 +141,8 @@ constexpr uint64_t kScatterThreads = 148 * 4 * 32 * 4;
 
 // --------------------------------------------------------------------------
 // storage vs compute.  Every MSM buffer (bases, partials, buckets, reduction items)
-// holds canonical values of Fq or Fq2.  Level 1 computes in FqL (G1, values below 2p)
-// and Fq2 (G2), the levels after it on quads of lanes (quad.cuh) in FqL and Fq2L, the
+// holds canonical values of Fq or Fq2.  Level 1 computes on values below 2p, in FqL (G1) and
+// Fq2M (G2), the levels after it on quads of lanes (quad.cuh) in FqL and Fq2L, the canonical
 // Fq2 product with two reductions instead of three.
 // --------------------------------------------------------------------------
 
@@ -305,7 +305,7 @@ struct SmXyzzFq {
     __device__ __forceinline__ static point load(const Affine<Fq> &p) { return lda(p); }
 };
 
-// G2: Fq2 coordinates (16 x 32-bit words), the library's Montgomery domain.
+// G2: Fq2M coordinates (16 words, each half below 2p).
 template <int BS>
 struct SmXyzzFq2 {
     using point = Affine<Fq2M>;

@@ -8,7 +8,7 @@
 //
 // Steps (all on the device, no host round trip):
 //  1. sort: each scalar leaves Montgomery form and is cut into W signed c-bit
-//     digits d in [-2^(c-1), 2^(c-1)]; bucket |d| - 1 receives the point
+//     digits d in [-(2^(c-1) - 1), 2^(c-1)]; bucket |d| - 1 receives the point
 //     (negated when d < 0).  Counts are histogrammed with warp-aggregated
 //     atomics, an exclusive scan gives bucket offsets, and a scatter writes
 //     (point, sign) entries in bucket order.  The sort depends only on the scalars and the
@@ -18,9 +18,10 @@
 //     [t K1, (t+1) K1) into XYZZ accumulators (mixed add 8M + 2S, with the
 //     doubling branch), one run per bucket it crosses, so all lanes do equal
 //     work whatever the bucket sizes.  A bucket spread over several segments
-//     leaves one partial per segment; a bucket of many pieces is finished by fix-up
-//     levels of fan-in 16, so one holding a large share of all points (repeated or
-//     small scalars) costs O(log n) sequential additions.
+//     leaves one partial per segment; up to 4 or 16 of them are added up by the bucket
+//     reduction, more by fix-up levels of fan-in 4 in one launch, so a bucket that holds a
+//     large share of all points (repeated or small scalars) costs O(log n) sequential
+//     additions.
 //  3. bucket reduction: sum_b (b + 1) S_b in levels of 64 items per block: a
 //     shared-memory suffix scan and tree sums make a level about 2 log2(block)
 //     dependent additions deep.  From the fix-up levels on four lanes hold a point
@@ -260,7 +261,7 @@ int msm_class_sort_run(MsmClassSort &s, const MsmDedup &d, const uint32_t *gathe
 // fix-up levels), normalised to affine as the bases of a small MSM over the
 // class values.
 struct MsmClassAcc {
-    MsmShape seg;      // n = the support's points, nb = kClassMax classes, k1, k2
+    MsmShape seg;      // n = the support's points, nb = kClassMax classes
     DevBuf partials, buckets, fix;
     MsmBases small;    // the class sums (affine; G2: and their psi images), non-folded
     MsmScratch small_s;

@@ -109,7 +109,7 @@ __global__ void k_group_op(int op, const F *a, const F *b, F *out, uint64_t n)
 }
 
 // Each thread runs 4 independent product chains; the result is stored so the
-// work cannot be eliminated.  variant 0: operator* (64-bit accumulation CIOS),
+// work cannot be eliminated.  variant 0: operator* (even and odd accumulators),
 // 1: mont_mul_cc (PTX carry-chain CIOS), 2: squaring; k_bench_mul52 below is
 // variant 3 (the 52-bit-limb FP64 product, canonical) and 4 (lazily reduced).
 constexpr int kBenchIters = 256;

@@ -16,12 +16,22 @@ constexpr size_t kOutOffset[kNumMsm] = {0, 96, 192, 288, 384}; // A, B1, L, H, B
 constexpr int kWitnessOrder[4] = {kMsmB2, kMsmA, kMsmB1, kMsmL};
 // Repeated witness values go through the class path (msm.cuh) only for circuits of more
 // variables than this.  It is a chain of some forty dependent small launches, which takes
-// longer than the additions that it saves in a small prove.  Measured, class path on / off,
-// one prove with blinding (batch of 8 proofs): poseidon of 4, 16 and 64 hashes (2^11, 2^13
-// and 2^15 variables) 1.97 / 0.96, 2.12 / 1.15 and 2.45 / 2.26 ms (4.10 / 1.64, 6.63 / 3.02
-// and 10.1 / 7.3 ms); 256 hashes (2^17) 3.47 / 4.73 ms (20.6 / 21.4 ms); 2,048 (2^20)
-// 10.0 / 17.2 ms.  Without repeated values the path only costs: matmul 32 (2^16)
-// 2.02 / 1.58 ms, sql-aggregate 256 (2^18) 8.78 / 7.71 ms.
+// longer than the additions that it saves in a small prove.  Measured, class path on / off in
+// ms, one prove with blinding (a batch of 8 proofs):
+//   variables, circuit            dense preimages          half                     sparse
+//   2^11 poseidon 4                                                                1.74 / 0.84 (4.30 / 1.67)
+//   2^13 poseidon 16                                                               2.18 / 1.02 (6.26 / 3.22)
+//   2^15 poseidon 64     2.28 / 1.59 (8.9 / 6.8)   2.49 / 1.64 (10.3 / 7.0)   2.29 / 1.62 (8.3 / 7.1)
+//   2^16 poseidon 128    2.86 / 2.10 (13.4 / 11.2) 3.01 / 2.13 (14.0 / 11.4)  2.61 / 2.14 (10.8 / 11.6)
+//   2^17 poseidon 256    3.41 / 3.11 (21.0 / 18.6)                            2.75 / 3.15 (14.3 / 19.1)
+//   2^20 poseidon 2,048                                                       10.0 / 17.2
+//   2^16 sql-aggregate 64 3.08 / 2.11 (14.4 / 11.2), 2^18 sql-aggregate 256 5.37 / 5.00 (35.7 / 33.1)
+//   2^16 matmul 32        1.28 / 1.23 (4.5 / 4.1),   2^17 matmul 40         2.24 / 2.20 (10.9 / 10.5)
+// The size stands in for the repetition, which decides and is only known on the device (of
+// the nonzero values of poseidon 128, 45,364 of 56,219 lie in classes with sparse preimages;
+// of poseidon 256 dense, 768 of 112,897).  Up to 2^16 variables the path gains in one of the
+// batches above only (7%) and costs up to twice the time; beyond it costs at most 13% where
+// little repeats.
 constexpr uint64_t kClassColsMin = uint64_t(1) << 16;
 
 } // namespace
