@@ -122,7 +122,8 @@ struct nkr_b200_msm_bases {
     nkr::DevBuf scalars;
     // events around a run and pinned memory for its result (192 B) and entry count: made
     // once, and the phase times are read when they are asked for; a run ends with one
-    // synchronisation (3,001 points 304 -> 276 us)
+    // synchronisation (3,001 points 304 -> 276 us).  The memory is a slot of the context's,
+    // or the handle's own when these are taken.
     cudaEvent_t ev[2] = {};
     uint8_t *result = nullptr;
     bool ran = false;
@@ -132,10 +133,11 @@ struct nkr_b200_msm_bases {
             if (e) cudaEventDestroy(e);
         for (auto e : ev)
             if (e) cudaEventDestroy(e);
-        if (result) cudaFreeHost(result);
+        if (result && !ctx->msm_results.give(result)) cudaFreeHost(result);
     }
 };
 constexpr size_t kMsmResultBytes = 192, kMsmCountAt = 192;
+static_assert(kMsmCountAt + 4 <= nkr::PinnedSlots::kBytes, "result slot size");
 
 using namespace nkr;
 
@@ -172,6 +174,7 @@ int nkr_b200_open(int device, nkr_b200_ctx **out)
         set_error("stream creation failed");
         return NKR_B200_ECUDA;
     }
+    ctx->msm_results.open();
     *out = ctx;
     return NKR_B200_OK;
 }
@@ -449,7 +452,9 @@ int nkr_b200_msm_bases_create(nkr_b200_ctx *ctx, int group, const void *bases, u
     NKR_TRY(msm_scratch_alloc(h->scratch, group, h->bases.shape));
     for (auto &e : h->scratch.acc.ev_acc) NKR_CUDA(cudaEventCreate(&e));
     for (auto &e : h->ev) NKR_CUDA(cudaEventCreate(&e));
-    if (cudaHostAlloc(reinterpret_cast<void **>(&h->result), kMsmResultBytes + 4, cudaHostAllocDefault) != cudaSuccess) {
+    h->result = ctx->msm_results.take();
+    if (!h->result &&
+        cudaHostAlloc(reinterpret_cast<void **>(&h->result), kMsmResultBytes + 4, cudaHostAllocDefault) != cudaSuccess) {
         cudaGetLastError();
         h->result = nullptr;
         set_error("pinned host allocation failed");

@@ -294,3 +294,38 @@ def test_statistics_of_runs(ctx, orc, rng, group):
         assert all(st[p] >= 0 for p in phases) and st["acc_ms"] > 0
         assert sum(st[p] for p in phases) <= st["total_ms"] + 5e-3  # 1 us of resolution a phase
     b.free()
+
+
+def test_many_handles_on_several_threads(orc, rng):
+    """More handles at once than the context has result slots, run from four threads, some of
+    them freed and made again: every run returns its own handle's sum."""
+    import threading
+    ctx = nk.Context(0)
+    gen = orc.g1_generator()
+    ks = O.random_fr(6, rng)
+    pts = np.stack([orc.mul_affine(1, gen, k) for k in ks])
+    handles = [nk.MsmBases(ctx, 1, O.affine_to_jac(1, np.roll(pts, i, axis=0))) for i in range(70)]
+    for i in range(0, 70, 3):
+        handles[i].free()
+        handles[i] = nk.MsmBases(ctx, 1, O.affine_to_jac(1, np.roll(pts, i, axis=0)))
+    kint = [O.fr_int(k) for k in ks]
+    bad = []
+
+    def work(t):
+        r = np.random.default_rng(t)
+        for i in list(range(t, 70, 4)) * 3:
+            s = r.integers(0, 1 << 30, 6)
+            got, _ = handles[i].run(np.stack([O.fr_mont(int(v)) for v in s]))
+            total = sum(int(v) * kint[(j - i) % 6] for j, v in enumerate(s)) % O.R
+            if not np.array_equal(got[:8], orc.mul_affine(1, gen, O.fr_mont(total))):
+                bad.append(i)
+
+    threads = [threading.Thread(target=work, args=(t,)) for t in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad
+    for h in handles:
+        h.free()
+    ctx.close()
