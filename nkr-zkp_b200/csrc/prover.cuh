@@ -6,16 +6,17 @@
 // A key holds what every proof of the circuit reads (CSR matrices, NTT tables,
 // folded MSM bases) once.  Everything one proof writes lives in a prove slot:
 // witness and quotient vectors, digit sorts, bucket scratch, result points,
-// five streams and their events, and a CUDA graph of the whole prove.  Slot 0
+// its streams and their events, and CUDA graphs of the whole prove.  Slot 0
 // serves nkr_b200_prove; batches and the request server add slots so several
 // proofs of one key are in flight at once.
 //
 // Streams of a slot: after the witness upload and the SpMV, the four witness
 // MSMs (a, b_g1, l on G1 and b_g2 on G2) run on their own streams while the
 // main stream computes H (7 transforms) and then the H MSM; the reference runs
-// every stage serially with a device sync after each.  The witness's repeated
-// values are found once per prove, and each witness MSM sums the bases of every
-// class of equal values on a class stream of higher priority (msm.cuh).
+// every stage serially with a device sync after each.  In circuits of more than 2^16
+// variables the witness's repeated values are found once per prove, and each witness MSM
+// sums the bases of every class of equal values on a class stream of higher priority
+// (msm.cuh).
 #pragma once
 
 #include <cstdint>
