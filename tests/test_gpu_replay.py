@@ -89,3 +89,46 @@ def test_stage_times_of_issued_and_replayed_proves(ctx, kind, param):
             assert tuple(be.stage_times().values()) == seen[-1]
     assert len(set(seen)) == 6  # every prove's own
     be.free()
+
+
+def test_threads_with_keys_of_their_own(ctx, orc):
+    """Four threads prove and blind on a key each, from the first prove over the capture to
+    replays, while this one allocates and runs MSMs and transforms on the same context."""
+    import threading
+    specs = [("poseidon", 2), ("poseidon", 20), ("matmul", 8), ("sql-aggregate", 8)]
+    keys, want = [], []
+    r, s = O.random_fr(2, np.random.default_rng(44))
+    for kind, param in specs:
+        r1, pk, be = _key(ctx, kind, param)
+        one = nk.Backend(ctx)
+        one.prepare(r1, pk)
+        raw = one.prove(r1.witness)
+        want.append((bytes(raw), bytes(one.blind(raw, r, s))))
+        one.free()
+        keys.append((be, r1.witness))
+    bad = []
+
+    def work(j):
+        be, w = keys[j]
+        try:
+            for i in range(8):
+                raw = be.prove(w)
+                if (bytes(raw), bytes(be.blind(raw, r, s))) != want[j]:
+                    bad.append((j, i))
+        except Exception as e:
+            bad.append((j, repr(e)))
+
+    rng = np.random.default_rng(45)
+    x, jac = O.random_fr(1 << 12, rng), np.tile(O.affine_to_jac(1, orc.g1_generator()[None]), (500, 1))
+    sc = O.random_fr(500, rng)
+    fft, msm = ctx.ntt(0, x), ctx.msm(1, jac, sc)
+    threads = [threading.Thread(target=work, args=(j,)) for j in range(4)]
+    for t in threads:
+        t.start()
+    while any(t.is_alive() for t in threads):
+        assert np.array_equal(ctx.ntt(0, x), fft) and np.array_equal(ctx.msm(1, jac, sc), msm)
+    for t in threads:
+        t.join()
+    assert not bad
+    for be, _ in keys:
+        be.free()
